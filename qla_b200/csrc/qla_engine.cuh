@@ -11,7 +11,7 @@
 // (`xX`, 4 B per site) stream their pointer/index tile through the same
 // pipeline and gather the records with per-thread read-only loads.
 //
-// A second, direct kernel (no staging) runs the gang-index `x` variants, whose
+// A second, warp-cooperative kernel runs the gang-index `x` variants, whose
 // every operand is scattered, and any call whose pointers are not 16-B
 // aligned (bulk copies require 16-B alignment).  Both kernels share the
 // per-site code, so their results are identical.
@@ -352,8 +352,175 @@ __global__ void __launch_bounds__(288) site_tma_kernel(const SiteParams p) {
 }
 
 // ---------------------------------------------------------------------------
-// Kernel 2: direct, grid-stride, one site per thread (gang-index variants and
-// unaligned operands).
+// Kernel 2: warp-cooperative, for the gang-index variants (every operand
+// scattered) and operands that a bulk copy cannot move (not 16-B aligned).
+//
+// A warp takes 32 sites at a time.  Its lanes copy the sites' records into
+// the warp's shared-memory slice with cp.async, piece by piece: consecutive
+// lanes take consecutive 16-B (or 8-B) pieces of one record, so one
+// instruction touches 4 to 10 records' lines instead of 32 (a thread reading
+// its own record makes every instruction touch 32 lines, and the L1 then
+// spends a cycle on each: that bound the one-site-per-thread form).  Then
+// each lane computes one site from shared memory, and results leave the same
+// way.  The gang index and the operands' pointers or indices of the next 32
+// sites are loaded while the records are in flight, which takes two of the
+// three dependent latencies out of the loop.  Shared record slots hold an odd
+// number of 16-B (8-B) units: conflict-free for one record per lane.
+// Measured, QLA_F3_D_xpeq_spproj_pMa_times_pD on the even sites of
+// 32^3 x 64: 142 us with one site per thread, 112 so (5.9-6.0 TB/s of
+// DRAM traffic: alternate records share their 64-B granules).
+template <int RB>
+struct CoopSlot {  // shared bytes of one record slot
+  static constexpr unsigned value = (RB % 16 == 0 && (RB / 16) % 2 == 0) ? RB + 16 : RB;
+};
+template <class OP>
+struct CoopLayout {
+  using R = typename OP::R;
+  static constexpr int C = (int)sizeof(Cx<R>);
+  static constexpr unsigned S0 = OP::NIN > 0 ? CoopSlot<OP::N0 * C>::value : 0,
+                            S1 = OP::NIN > 1 ? CoopSlot<OP::N1 * C>::value : 0,
+                            S2 = OP::NIN > 2 ? CoopSlot<OP::N2 * C>::value : 0,
+                            SO = OP::NOUT > 0 ? CoopSlot<OP::NOUT * C>::value : 0;
+  static constexpr unsigned o1 = 32 * S0, o2 = o1 + 32 * S1, oo = o2 + 32 * S2;
+  static constexpr unsigned warp_bytes = oo + 32 * SO;  // each part is a multiple of 256 B
+};
+
+// address of operand o's record of site k
+template <class OP, int N>
+__device__ __forceinline__ const char* rec_addr(const Opnd& o, long long k) {
+  constexpr int RB = N * (int)sizeof(Cx<typename OP::R>);
+  if (o.mode == OM_PTR) return static_cast<const char*>(o.ptrs[k]);
+  return static_cast<const char*>(o.base) + (o.mode == OM_IDX ? (long long)o.idx[k] : k) * RB;
+}
+
+// Walk over the pieces of 32 records (P pieces each), a piece per lane:
+// f(record, piece, live).  Records of up to 16 pieces go 32 / P at a time, so
+// that a lane keeps its piece number and its addresses advance by constants;
+// longer records in one run.  Every lane makes every call, so f may shuffle.
+// (The empty asm keeps the offsets from being held in registers across the
+// site loop.)
+template <int P, class F>
+__device__ __forceinline__ void for_pieces(int lane, F&& f) {
+  asm volatile("" : "+r"(lane));
+  if constexpr (P <= 16) {
+    constexpr int G = 32 / P, ITS = (32 + G - 1) / G;
+    const int r0 = lane / P, pc = lane - r0 * P;
+#pragma unroll
+    for (int it = 0; it < ITS; it++) f(it * G + r0, pc, r0 < G);
+  } else {
+#pragma unroll 4
+    for (int it = 0; it < P; it++) {
+      const int q = it * 32 + lane;
+      f(q / P, q % P, true);
+    }
+  }
+}
+
+// copies the records at `addr` (one per lane, the first nv lanes valid) into slots
+template <int RB>
+__device__ __forceinline__ void coop_fetch(unsigned char* slots, const char* addr, int nv, int lane) {
+  constexpr unsigned SL = CoopSlot<RB>::value;
+  const unsigned long long a = reinterpret_cast<unsigned long long>(addr);
+  const bool wide = RB % 16 == 0 && __all_sync(0xffffffffu, lane >= nv || (a & 15u) == 0);
+  if (wide) {
+    for_pieces<(RB % 16 == 0 ? RB / 16 : 1)>(lane, [&](int r, int pc, bool live) {
+      const char* src = reinterpret_cast<const char*>(__shfl_sync(0xffffffffu, a, r & 31)) + pc * 16;
+      if (live && r < nv) cp_async_16(slots + r * SL + pc * 16, src);
+    });
+  } else {
+    for_pieces<RB / 8>(lane, [&](int r, int pc, bool live) {
+      const char* src = reinterpret_cast<const char*>(__shfl_sync(0xffffffffu, a, r & 31)) + pc * 8;
+      if (live && r < nv) cp_async_8(slots + r * SL + pc * 8, src);
+    });
+  }
+}
+
+// writes the records in the slots to `addr` (one per lane)
+template <int RB>
+__device__ __forceinline__ void coop_store(const unsigned char* slots, char* addr, int nv, int lane) {
+  constexpr unsigned SL = CoopSlot<RB>::value;
+  const unsigned long long a = reinterpret_cast<unsigned long long>(addr);
+  const bool wide = RB % 16 == 0 && __all_sync(0xffffffffu, lane >= nv || (a & 15u) == 0);
+  if (wide) {
+    for_pieces<(RB % 16 == 0 ? RB / 16 : 1)>(lane, [&](int r, int pc, bool live) {
+      char* dst = reinterpret_cast<char*>(__shfl_sync(0xffffffffu, a, r & 31)) + pc * 16;
+      if (live && r < nv) *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(slots + r * SL + pc * 16);
+    });
+  } else {
+    for_pieces<RB / 8>(lane, [&](int r, int pc, bool live) {
+      char* dst = reinterpret_cast<char*>(__shfl_sync(0xffffffffu, a, r & 31)) + pc * 8;
+      if (live && r < nv) *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(slots + r * SL + pc * 8);
+    });
+  }
+}
+
+template <class OP>
+__global__ void __launch_bounds__(128) site_coop_kernel(const SiteParams p) {
+  using R = typename OP::R;
+  using L = CoopLayout<OP>;
+  constexpr int NA = ArrN<OP::NACC>::value, C = (int)sizeof(Cx<R>);
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  unsigned char* sl = smem + (size_t)warp * L::warp_bytes;
+  DD dacc[NA];
+#pragma unroll
+  for (int a = 0; a < NA; a++) dacc[a] = DD{0.0, 0.0};
+  const long long step = (long long)gridDim.x * nw * 32;
+  const char *a0 = nullptr, *a1 = nullptr, *a2 = nullptr;
+  char* ao = nullptr;
+  auto addresses = [&](long long i) {  // this lane's record addresses for loop position i
+    if (i >= p.n) return;
+    const long long k = p.gang ? (long long)p.gang[i] : i;
+    if constexpr (OP::NIN > 0) a0 = rec_addr<OP, OP::N0>(p.in[0], k);
+    if constexpr (OP::NIN > 1) a1 = rec_addr<OP, OP::N1>(p.in[1], k);
+    if constexpr (OP::NIN > 2) a2 = rec_addr<OP, OP::N2>(p.in[2], k);
+    if constexpr (OP::NOUT > 0) ao = static_cast<char*>(p.out) + k * (OP::NOUT * C);
+  };
+  long long i0 = ((long long)blockIdx.x * nw + warp) * 32;
+  addresses(i0 + lane);
+  for (; i0 < p.n; i0 += step) {
+    const int nv = p.n - i0 < 32 ? (int)(p.n - i0) : 32;
+    if constexpr (OP::NIN > 0) coop_fetch<OP::N0 * C>(sl, a0, nv, lane);
+    if constexpr (OP::NIN > 1) coop_fetch<OP::N1 * C>(sl + L::o1, a1, nv, lane);
+    if constexpr (OP::NIN > 2) coop_fetch<OP::N2 * C>(sl + L::o2, a2, nv, lane);
+    char* dst = ao;
+    if constexpr (OP::NOUT > 0) {
+      if (p.out_read) coop_fetch<OP::NOUT * C>(sl + L::oo, ao, nv, lane);
+    }
+    addresses(i0 + step + lane);
+    cp_async_wait_all();
+    __syncwarp();
+    if (lane < nv) {
+      Cx<R> x0[ArrN<OP::N0>::value], x1[ArrN<OP::N1>::value], x2[ArrN<OP::N2>::value];
+      if constexpr (OP::NIN > 0) load_rec<R, ArrN<OP::N0>::value>(x0, sl + lane * L::S0);
+      if constexpr (OP::NIN > 1) load_rec<R, ArrN<OP::N1>::value>(x1, sl + L::o1 + lane * L::S1);
+      if constexpr (OP::NIN > 2) load_rec<R, ArrN<OP::N2>::value>(x2, sl + L::o2 + lane * L::S2);
+      if constexpr (OP::NOUT > 0) {
+        Cx<R> y[OP::NOUT];
+        if (p.out_read) {
+          load_rec<R, OP::NOUT>(y, sl + L::oo + lane * L::SO);
+        } else {  // (undefined, it would stay live around the loop)
+#pragma unroll
+          for (int e = 0; e < OP::NOUT; e++) y[e] = Cx<R>{R(0), R(0)};
+        }
+        OP::apply(p, x0, x1, x2, y);
+        store_rec_smem<R, OP::NOUT>(sl + L::oo + lane * L::SO, y);
+      } else {
+        double acc[NA];
+        OP::accum(p, x0, x1, x2, acc);
+        acc_fold<OP>(dacc, acc);
+      }
+    }
+    __syncwarp();  // results in the slots; every lane is done with the inputs
+    if constexpr (OP::NOUT > 0) {
+      coop_store<OP::NOUT * C>(sl + L::oo, dst, nv, lane);
+      __syncwarp();  // the slots are free for the next 32 sites
+    }
+  }
+  if constexpr (OP::NACC > 0) reduce_finish<OP>(p, dacc);
+}
+
+// One site per thread, for the allocation-free entry point's unaligned calls.
 template <class OP>
 __global__ void __launch_bounds__(256) site_direct_kernel(const SiteParams p) {
   constexpr int NA = ArrN<OP::NACC>::value;

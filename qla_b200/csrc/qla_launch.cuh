@@ -1,5 +1,5 @@
 // qla_launch.cuh -- host-side launch of an engine OP: path selection (bulk-copy
-// pipeline vs direct), tile shape, occupancy-sized persistent grid, reduction
+// pipeline or warp-cooperative kernel), tile shape, occupancy-sized persistent grid, reduction
 // scratch and the synchronous host-result semantics of the reference.
 #pragma once
 #include <cstring>
@@ -113,12 +113,23 @@ struct SiteLauncher {
     }
 
     if (direct) {
-      const int threads = 256;
-      long long want = (p.n + threads - 1) / threads;
-      long long cap = (long long)sms * 8;
-      int grid = (int)(want < cap ? want : cap);
-      if (grid < 1) grid = 1;
-      site_direct_kernel<OP><<<grid, threads, 0, st>>>(p);
+      // four warps a block, fewer where their slices would leave less than
+      // four blocks an SM
+      constexpr unsigned wb = CoopLayout<OP>::warp_bytes;
+      int nw = 4;
+      while (nw > 1 && nw * wb > 48u * 1024u) nw /= 2;
+      const size_t smem = (size_t)nw * wb;
+      const void* fn = reinterpret_cast<const void*>(&site_coop_kernel<OP>);
+      set_smem_attr(fn, smem);
+      long long grid = (p.n + 32 * nw - 1) / (32 * nw);
+      const long long cap = (long long)blocks_per_sm(fn, 32 * nw, smem) * sms;
+      if (grid > cap) grid = cap;
+      if (reduce && grid > rs->max_blocks) grid = rs->max_blocks;
+      void* args[] = {&p};
+      if (cudaLaunchKernel(fn, dim3((unsigned)grid), dim3(32u * nw), args, smem, st) != cudaSuccess) {
+        check_launch(kernel_id);
+        return;
+      }
     } else {
       unsigned bps = 0;
       for (int j = 0; j < OP::NIN; j++)
