@@ -4,26 +4,26 @@
 // A lattice code often applies a short level-1 sequence to many independent
 // fields (sub-lattices, sources, time slices).  Launching QLA's functions
 // once per field and step costs a launch each and leaves the GPU idle on the
-// small fields.  Here a plan flattens every field's tiles into one global
-// tile list (prefix sums over per-field tile counts) and one persistent,
-// warp-specialised bulk-copy pipeline walks that list.  Each field carries a
-// small program (qlagpu_F3_batch_program): streams (its record arrays, some
-// gathered through an int32 index) and steps drawn from the engine's per-site
-// operators -- colour-matrix left multiplication (lmult_site), spin
-// projection and reconstruction (the SpprojOp / SpreconOp bodies), real
-// multiples and copies -- so a field's results are bit-identical to the
-// separate QLA_F3 calls the steps stand for.
+// small fields.  Here a plan cuts every field into tiles of 32 sites and deals
+// the tiles to the warps of one persistent launch, in contiguous runs of equal
+// estimated cost.  Each field carries a small program (qlagpu_F3_batch_program):
+// streams (its record arrays, some gathered through an int32 index) and steps
+// drawn from the engine's per-site operators -- colour-matrix left
+// multiplication (lmult_site), spin projection and reconstruction (the
+// SpprojOp / SpreconOp bodies), real multiples and copies -- so a field's
+// results are bit-identical to the separate QLA_F3 calls the steps stand for.
 //
-// Per tile the producer lane copies, with 1-D bulk copies into the next
-// pipeline stage, every contiguous input stream of the field, the index tile
-// of every gathered stream and the old values of every INOUT stream.  The
-// consumer warps run the program one site per lane: operands come from the
-// stage, from gathers (read-only global loads at the staged index) or from
-// two per-site registers; stored results go through a per-warp
-// per-warp shared slice and one bulk store per output stream.  Steps
-// only see values of the same site, so sites are independent and the launch
-// needs no grid-wide ordering.  Partial tiles, and fields whose arrays are
-// not 16-B aligned, run the same program with plain loads and stores.
+// Every warp runs by itself, with no block-wide synchronisation: it brings the
+// next tile's records into shared memory while it computes the present one
+// (bulk copies; gathered V and M records, whose length no bulk copy takes,
+// with cp.async), and the index tile of the tile after that.  Then each lane
+// takes one site through the field's steps.  Every value a step reads or makes
+// (stream records, registers, stored results) has a fixed shared-memory slot,
+// chosen by the planner, so a step is one call of a routine compiled for its
+// operation and record kinds, chosen by a uniform switch, with nothing kept in
+// registers between steps.  Stored results leave by one bulk store per stream.
+// Partial tiles and fields whose arrays are only 8-B aligned run the same
+// steps with 8-B copies.
 //
 // The launch (qlagpu_batch_run) passes only the plan's device table: it can
 // be replayed from a captured CUDA graph.
@@ -51,19 +51,20 @@ __host__ __device__ constexpr int kncplx(int kind) { return kind == BK_V ? 3 : k
 struct BStream {
   char* base;
   const int* idx;
-  long long nsrc;
   int kind, role;
-  unsigned stage_off;  // contiguous IN / INOUT: record tile; gathered IN: index tile
-  unsigned out_off;    // OUT / INOUT: this stream's part of a warp's output slice
+  unsigned lim;       // gathered: indices must lie in [0, lim); 0: unchecked
+  int wide;           // records start on 16-B boundaries
+  int used;           // some step reads it (IN / INOUT: it is copied in)
+  unsigned slot;      // IN / INOUT: its records' place in the stage
+  unsigned idx_slot;  // gathered: three index tiles in the warp's fixed area
+  unsigned out;       // OUT / INOUT: the stored result's place in the stage
 };
-
 struct BStep {
-  int op, eqop, a, b, dst, store, adja, adjb, mu, sign;
-  int kind_a, kind_b, kind_r;  // operand and result kinds (checked on the host)
-  int load_stream;             // peq / meq: the old value comes from this INOUT stream's tile, else -1
-  int spill;                   // a later step other than the next one reads this result's register
-  int src_a, src_b;            // SrcKind of the operands (classified by the planner)
+  int code;  // StepCode
+  int eqop, mu, sign;
+  unsigned a, b, old, res;  // places in the stage of the operands, of the value that peq / meq update, and of the result
   float r;
+  int pad;
 };
 
 struct alignas(16) BField {
@@ -71,699 +72,415 @@ struct alignas(16) BField {
   BStep st[kMaxSteps];
   int nstreams, nsteps;
   long long n, tile0;
-  unsigned tx_bytes;  // bytes the producer copies per full tile
-  int direct;         // some base not 16-B aligned: every tile by plain loads
-  int shape;          // ShapeId of this field's program (SH_GENERIC: none of the catalogue)
+  int bulk;            // every contiguous array that is read or written starts on a 16-B boundary
+  unsigned tx;         // bytes the contiguous streams of a full tile bring
+  int ngather;         // gathered streams that some step reads
+  int gather[kMaxStreams];
 };
 
 struct BatchParams {
   const BField* fields;
+  const long long* start;  // first tile of each run, and the end; block b takes runs b, b + grid, ...
+  int runs;
   int nfields;
-  long long ntiles;
-  int stages;
-  unsigned stage_bytes, out_slice_bytes;  // out slice: 32 sites of every output stream
-  int spill_regs;                         // some program keeps a register in shared memory
-  long long chunk;                        // consecutive tiles per group dealt to a block
+  unsigned fixed_bytes, stage_bytes, warp_bytes;
+  int stages;              // 1 or 2
   unsigned* err;
 };
 
 struct BatchPlan {
-  BField* dfields;
-  int nfields;
+  BField* dfields;    // device: the field table, then the runs' first tiles
+  long long* dstart;
+  int nfields, threads, grid, stages, runs;
   long long ntiles;
-  int threads, stages, grid;
-  unsigned stage_bytes, out_slice_bytes;
-  int spill_regs;
-  long long chunk;  // see BatchParams
-  int mc;     // record capacity of the kernel instance: 9 or 12 complex numbers
-  int shape;  // ShapeId of the kernel instance (SH_GENERIC: the interpreter)
+  unsigned fixed_bytes, stage_bytes, warp_bytes;
   size_t smem;
 };
 
-// The field of tile g given the previous answer f (or -1): tiles come in
-// runs, so a range check usually settles it without the search.
-__device__ __forceinline__ int find_field(const long long* tile0, int nf, long long g);
-__device__ __forceinline__ int field_of(const long long* tile0, int nf, long long g, int f) {
-  if (f >= 0 && tile0[f] <= g && (f + 1 == nf || g < tile0[f + 1])) return f;
-  return find_field(tile0, nf, g);
+// The routine of a step: LMULT by the kind of b and the adjoints, then the
+// other operations by their record kind.
+enum StepCode : int { SC_LMULT = 0, SC_SPPROJ = 16, SC_SPRECON = 17, SC_RTIMES = 20, SC_COPY = 24 };
+
+constexpr int kDescWords = (int)((sizeof(BField) + 15) / 16);  // 16-B words
+
+// bytes of one record, and of its shared slot
+__host__ __device__ constexpr unsigned rec_b(int kind) { return (unsigned)kncplx(kind) * 8u; }
+
+
+// --- copies between global memory and a warp's slots with plain instructions:
+// partial tiles, and fields that are not 16-B aligned
+__device__ __forceinline__ void run_in(unsigned char* dst, const char* src, unsigned bytes, int lane) {
+#pragma unroll 1
+  for (unsigned o = lane * 8u; o < bytes; o += 256u) cp_async_8(dst + o, src + o);
 }
-__device__ __forceinline__ int find_field(const long long* tile0, int nf, long long g) {
-  int lo = 0, hi = nf - 1;  // last field with tile0 <= g
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (tile0[mid] <= g)
-      lo = mid;
-    else
-      hi = mid - 1;
-  }
-  return lo;
+__device__ __forceinline__ void run_out(char* dst, const unsigned char* src, unsigned bytes, int lane) {
+#pragma unroll 1
+  for (unsigned o = lane * 8u; o < bytes; o += 256u)
+    *reinterpret_cast<uint2*>(dst + o) = *reinterpret_cast<const uint2*>(src + o);
 }
-
-// One record of any kind the plan uses, MC complex numbers long: 12 when
-// some field uses DiracFermions, else 9 (colour matrices are the longest),
-// which keeps the kernel's registers down for V / H / M programs.
-template <int MC>
-using Rec = Cx<float>[MC];
-
-
-// --- record movement with a compile-time length N (complex numbers)
-template <int N, int MC>
-__device__ __forceinline__ void ld_smem(Rec<MC>& x, const unsigned char* p) {
-  if constexpr (N % 2 == 0) {  // H, D: 16-B multiples
-    const float4* q = reinterpret_cast<const float4*>(p);
+// a gathered tile: P 8-B pieces per record, 32 / P records at a time, one lane
+// per piece (a lane keeps its piece number, so its addresses advance by
+// constants); nv records, record r at index idx[r]; the records of the lanes in
+// `bad` read zero
+template <int P>
+__device__ __forceinline__ void gather_pieces(unsigned char* dst, const char* base, const int* idx, int nv,
+                                              unsigned bad, int lane) {
+  constexpr int G = 32 / P, ITS = (32 + G - 1) / G;
+  const int r0 = lane / P, pc = lane - r0 * P;
+  if (r0 >= G) return;
+  const char* from = base + pc * 8;
+  dst += (r0 * P + pc) * 8;
+  idx += r0;
+  if (nv == 32 && bad == 0u) {
 #pragma unroll
-    for (int e = 0; e < N / 2; e++) {
-      const float4 v = q[e];
-      x[2 * e] = Cx<float>{v.x, v.y};
-      x[2 * e + 1] = Cx<float>{v.z, v.w};
-    }
+    for (int it = 0; it < ITS; it++)
+      if ((it + 1) * G <= 32 || r0 < 32 - it * G)
+        cp_async_8(dst + it * G * P * 8, from + (long long)idx[it * G] * (P * 8));
   } else {
-    const float2* q = reinterpret_cast<const float2*>(p);
-#pragma unroll
-    for (int e = 0; e < N; e++) {
-      const float2 v = q[e];
-      x[e] = Cx<float>{v.x, v.y};
+#pragma unroll 1
+    for (int it = 0; it < ITS; it++) {
+      const int r = it * G + r0;
+      if (r >= nv) break;
+      if ((bad >> r) & 1u)
+        *reinterpret_cast<uint2*>(dst + it * G * P * 8) = make_uint2(0u, 0u);
+      else
+        cp_async_8(dst + it * G * P * 8, from + (long long)idx[it * G] * (P * 8));
     }
   }
 }
-template <int N, int MC>
-__device__ __forceinline__ void st_smem(unsigned char* p, const Rec<MC>& y) {
-  if constexpr (N % 2 == 0) {
-    float4* q = reinterpret_cast<float4*>(p);
-#pragma unroll
-    for (int e = 0; e < N / 2; e++) q[e] = make_float4(y[2 * e].re, y[2 * e].im, y[2 * e + 1].re, y[2 * e + 1].im);
-  } else {
-    float2* q = reinterpret_cast<float2*>(p);
-#pragma unroll
-    for (int e = 0; e < N; e++) q[e] = make_float2(y[e].re, y[e].im);
-  }
+
+// --- one record of this lane, in its slot
+template <int N>
+__device__ __forceinline__ void ld_slot(Cx<float> (&x)[N], const unsigned char* p) {
+  load_rec<float, N>(x, p);
 }
-template <int N, int MC>
-__device__ __forceinline__ void ld_global(Rec<MC>& x, const void* p) {
-  const float2* q = reinterpret_cast<const float2*>(p);
-#pragma unroll
-  for (int e = 0; e < N; e++) {
-    const float2 v = __ldg(q + e);
-    x[e] = Cx<float>{v.x, v.y};
-  }
-}
-template <int N, int MC>
-__device__ __forceinline__ void ld_global_rw(Rec<MC>& x, const void* p) {  // a stream this launch also writes
-  const float2* q = reinterpret_cast<const float2*>(p);
-#pragma unroll
-  for (int e = 0; e < N; e++) {
-    const float2 v = q[e];
-    x[e] = Cx<float>{v.x, v.y};
-  }
-}
-template <int N, int MC>
-__device__ __forceinline__ void st_global(void* p, const Rec<MC>& y) {
-  float2* q = reinterpret_cast<float2*>(p);
-#pragma unroll
-  for (int e = 0; e < N; e++) q[e] = make_float2(y[e].re, y[e].im);
-}
-template <int MC>
-__device__ __forceinline__ void zero_rec(Rec<MC>& x) {
-#pragma unroll
-  for (int e = 0; e < MC; e++) x[e] = Cx<float>{0.f, 0.f};
-}
-template <int MC>
-__device__ __forceinline__ void copy_rec(Rec<MC>& x, const Rec<MC>& y) {
-#pragma unroll
-  for (int e = 0; e < MC; e++) x[e] = y[e];
-}
-template <int N, int MC>  // the first N complex numbers only
-__device__ __forceinline__ void copy_rec_n(Rec<MC>& x, const Rec<MC>& y) {
-#pragma unroll
-  for (int e = 0; e < N; e++) x[e] = y[e];
+template <int N>
+__device__ __forceinline__ void st_slot(unsigned char* p, const Cx<float> (&y)[N]) {
+  store_rec_smem<float, N>(p, y);
 }
 
-// Where one site's operands live: the staged tile (stage != nullptr, lane
-// t) or global memory (site i).  Step registers: the previous step's result
-// stays in registers (`prev`); a result that a later, non-adjacent step reads
-// is also kept in shared memory, element-major (element e of register k of
-// thread t at regs + ((k * 12 + e) * T + t) * 8), so a warp touches
-// consecutive words.
-struct SiteSrc {
-  const unsigned char* stage;
-  int t;
-  long long i;
-  unsigned* err;
-  unsigned char* regs;
-  int T;
+// (a destination that no eqop reads is zeroed: left undefined, each routine's
+// array would stay live around the step loop and the kernel take 255 registers)
+template <int N>
+__device__ __forceinline__ void zero_slot(Cx<float> (&x)[N]) {
+#pragma unroll
+  for (int e = 0; e < N; e++) x[e] = Cx<float>{0.f, 0.f};
+}
+
+// this lane's record of kind K at place `off` of the stage
+struct Slots {
+  unsigned char* stage;
+  int lane;
+  template <int K>
+  __device__ __forceinline__ unsigned char* at(unsigned off) const {
+    return stage + off + (unsigned)lane * rec_b(K);
+  }
 };
-template <int N, int MC>
-__device__ __forceinline__ void reg_load(Rec<MC>& x, const SiteSrc& src, int slot) {
-  const float2* q = reinterpret_cast<const float2*>(src.regs) + (size_t)slot * 12 * src.T + src.t;
-#pragma unroll
-  for (int e = 0; e < N; e++) {
-    const float2 v = q[(size_t)e * src.T];
-    x[e] = Cx<float>{v.x, v.y};
-  }
-}
-template <int N, int MC>
-__device__ __forceinline__ void reg_store(const SiteSrc& src, int slot, const Rec<MC>& y) {
-  float2* q = reinterpret_cast<float2*>(src.regs) + (size_t)slot * 12 * src.T + src.t;
-#pragma unroll
-  for (int e = 0; e < N; e++) q[(size_t)e * src.T] = make_float2(y[e].re, y[e].im);
+// A step's result may take the place of a value that has been read for the
+// last time, of another record length: every lane has its operands in
+// registers before any lane stores.
+template <int K, int N>
+__device__ __forceinline__ void put(const Slots& sl, unsigned off, const Cx<float> (&y)[N]) {
+  __syncwarp();
+  st_slot(sl.at<K>(off), y);
+  __syncwarp();
 }
 
-// record of stream S at this site, as an input (gathered through its index)
-template <int N, int MC>
-__device__ __forceinline__ void fetch_stream(Rec<MC>& x, const BStream& S, const SiteSrc& src) {
-  if (S.idx) {
-    long long j = src.stage ? reinterpret_cast<const int*>(src.stage + S.stage_off)[src.t] : S.idx[src.i];
-    if (S.nsrc > 0 && (j < 0 || j >= S.nsrc)) {
-      raise_dev_error(src.err, QLA_DEVERR_BAD_INDEX);
-      zero_rec(x);
-      return;
-    }
-    ld_global<N>(x, S.base + j * (long long)(N * 8));
-  } else if (src.stage) {
-    ld_smem<N>(x, src.stage + S.stage_off + (unsigned)src.t * (N * 8));
-  } else if (S.role == BR_INOUT) {
-    ld_global_rw<N>(x, S.base + src.i * (N * 8));
-  } else {
-    ld_global<N>(x, S.base + src.i * (N * 8));
-  }
-}
-// operand `ref` (a stream, or a register) of kind `kind`; prev / prev_reg:
-// the previous step's result and its register
-template <int N, int MC>
-__device__ __forceinline__ void fetch_n(Rec<MC>& x, int ref, const BField& F, const SiteSrc& src,
-                                        const Rec<MC>& prev, int prev_reg) {
-  if (ref == prev_reg)
-    copy_rec(x, prev);
-  else if (ref >= kReg0)
-    reg_load<N>(x, src, ref - kReg0);
+// --- the steps (the engine's per-site operators).  The eqop is uniform: it is
+// branched on once per step, outside the element loops.
+template <int K, bool ADJA, bool ADJB>
+__device__ __forceinline__ void step_lmult(const BStep& S, const Slots& sl) {
+  constexpr int NCOL = K == BK_V ? 1 : K == BK_H ? 2 : K == BK_D ? 4 : 3, N = 3 * NCOL;
+  const bool load = (S.eqop == PEQ || S.eqop == MEQ);
+  Cx<float> a[9], b[N], y[N];
+  ld_slot(a, sl.at<BK_M>(S.a));
+  ld_slot(b, sl.at<K>(S.b));
+  if (load) ld_slot(y, sl.at<K>(S.old));
+  else zero_slot(y);
+  // y (0, or the old value) plus or minus a b
+  if (S.eqop == EQ || S.eqop == PEQ)
+    lmult_site<float, 3, NCOL, ADJA, ADJB>(PEQ, true, a, b, y);
   else
-    fetch_stream<N>(x, F.s[ref], src);
+    lmult_site<float, 3, NCOL, ADJA, ADJB>(MEQ, true, a, b, y);
+  put<K>(sl, S.res, y);
 }
-template <int MC>
-__device__ __forceinline__ void fetch(Rec<MC>& x, int ref, int kind, const BField& F, const SiteSrc& src,
-                                      const Rec<MC>& prev, int prev_reg) {
-  switch (kind) {
-    case BK_V: fetch_n<3>(x, ref, F, src, prev, prev_reg); break;
-    case BK_H: fetch_n<6>(x, ref, F, src, prev, prev_reg); break;
-    case BK_M: fetch_n<9>(x, ref, F, src, prev, prev_reg); break;
-    default:
-      if constexpr (MC >= 12) fetch_n<12>(x, ref, F, src, prev, prev_reg);
-      break;
-  }
+// F's body for (mu, sign), its eqop known at compile time where it is the usual one
+template <class F, int LA, int LY>
+__device__ __forceinline__ void step_spin(const BStep& S, const Cx<float> (&a)[LA], Cx<float> (&y)[LY]) {
+  if (S.eqop == EQ)
+    mu_sign_dispatch<F>(S.mu, S.sign, (int)EQ, a, y);
+  else if (S.eqop == PEQ)
+    mu_sign_dispatch<F>(S.mu, S.sign, (int)PEQ, a, y);
+  else
+    mu_sign_dispatch<F>(S.mu, S.sign, S.eqop, a, y);
 }
-template <int MC>
-__device__ __forceinline__ void set_reg(const SiteSrc& src, int slot, int kind, const Rec<MC>& y) {
-  switch (kind) {
-    case BK_V: reg_store<3>(src, slot, y); break;
-    case BK_H: reg_store<6>(src, slot, y); break;
-    case BK_M: reg_store<9>(src, slot, y); break;
-    default:
-      if constexpr (MC >= 12) reg_store<12>(src, slot, y);
-      break;
-  }
+__device__ __forceinline__ void step_spproj(const BStep& S, const Slots& sl) {
+  Cx<float> a[12], y[6];
+  ld_slot(a, sl.at<BK_D>(S.a));
+  if (S.eqop == PEQ || S.eqop == MEQ) ld_slot(y, sl.at<BK_H>(S.old));
+  else zero_slot(y);
+  step_spin<SpprojOp<float, 3>::Body>(S, a, y);
+  put<BK_H>(sl, S.res, y);
 }
-
-// --- the per-site arithmetic of each step kind (the engine's operators)
-template <int N, int MC>
-__device__ __forceinline__ void rtimes_n(int eqop, float at, const Rec<MC>& b, Rec<MC>& y) {  // RTimesOp
+__device__ __forceinline__ void step_sprecon(const BStep& S, const Slots& sl) {
+  Cx<float> h[6], y[12];
+  ld_slot(h, sl.at<BK_H>(S.a));
+  if (S.eqop == PEQ || S.eqop == MEQ) ld_slot(y, sl.at<BK_D>(S.old));
+  else zero_slot(y);
+  step_spin<SpreconOp<float, 3>::Body>(S, h, y);
+  put<BK_D>(sl, S.res, y);
+}
+template <int K, bool RTIMES>  // RTimesOp, CopyOp
+__device__ __forceinline__ void step_map(const BStep& S, const Slots& sl) {
+  constexpr int N = kncplx(K);
+  Cx<float> b[N], y[N];
+  ld_slot(b, sl.at<K>(S.a));
+  if (S.eqop == PEQ || S.eqop == MEQ) ld_slot(y, sl.at<K>(S.old));
+  else zero_slot(y);
 #pragma unroll
   for (int e = 0; e < N; e++) {
-    const float pr = rmul(at, b[e].re), pi = rmul(at, b[e].im);
-    switch (eqop) {
+    const float pr = RTIMES ? rmul(S.r, b[e].re) : b[e].re, pi = RTIMES ? rmul(S.r, b[e].im) : b[e].im;
+    switch (S.eqop) {
       case EQ: y[e].re = pr; y[e].im = pi; break;
       case EQM: y[e].re = -pr; y[e].im = -pi; break;
       case PEQ: y[e].re = radd(y[e].re, pr); y[e].im = radd(y[e].im, pi); break;
       default: y[e].re = rsub(y[e].re, pr); y[e].im = rsub(y[e].im, pi); break;
     }
   }
+  put<K>(sl, S.res, y);
 }
-template <int N, int MC>
-__device__ __forceinline__ void copy_n(int eqop, const Rec<MC>& b, Rec<MC>& y) {  // CopyOp
-#pragma unroll
-  for (int e = 0; e < N; e++) {
-    switch (eqop) {
-      case EQ: y[e] = b[e]; break;
-      case EQM: y[e].re = -b[e].re; y[e].im = -b[e].im; break;
-      case PEQ: y[e].re = radd(y[e].re, b[e].re); y[e].im = radd(y[e].im, b[e].im); break;
-      default: y[e].re = rsub(y[e].re, b[e].re); y[e].im = rsub(y[e].im, b[e].im); break;
+
+__device__ __forceinline__ void run_step(const BStep& S, const Slots& sl) {
+  switch (S.code) {
+    case SC_LMULT + BK_V * 4 + 0: step_lmult<BK_V, false, false>(S, sl); break;
+    case SC_LMULT + BK_V * 4 + 2: step_lmult<BK_V, true, false>(S, sl); break;
+    case SC_LMULT + BK_H * 4 + 0: step_lmult<BK_H, false, false>(S, sl); break;
+    case SC_LMULT + BK_H * 4 + 2: step_lmult<BK_H, true, false>(S, sl); break;
+    case SC_LMULT + BK_D * 4 + 0: step_lmult<BK_D, false, false>(S, sl); break;
+    case SC_LMULT + BK_D * 4 + 2: step_lmult<BK_D, true, false>(S, sl); break;
+    case SC_LMULT + BK_M * 4 + 0: step_lmult<BK_M, false, false>(S, sl); break;
+    case SC_LMULT + BK_M * 4 + 1: step_lmult<BK_M, false, true>(S, sl); break;
+    case SC_LMULT + BK_M * 4 + 2: step_lmult<BK_M, true, false>(S, sl); break;
+    case SC_LMULT + BK_M * 4 + 3: step_lmult<BK_M, true, true>(S, sl); break;
+    case SC_SPPROJ: step_spproj(S, sl); break;
+    case SC_SPRECON: step_sprecon(S, sl); break;
+    case SC_RTIMES + BK_V: step_map<BK_V, true>(S, sl); break;
+    case SC_RTIMES + BK_H: step_map<BK_H, true>(S, sl); break;
+    case SC_RTIMES + BK_D: step_map<BK_D, true>(S, sl); break;
+    case SC_RTIMES + BK_M: step_map<BK_M, true>(S, sl); break;
+    case SC_COPY + BK_V: step_map<BK_V, false>(S, sl); break;
+    case SC_COPY + BK_H: step_map<BK_H, false>(S, sl); break;
+    case SC_COPY + BK_D: step_map<BK_D, false>(S, sl); break;
+    default: step_map<BK_M, false>(S, sl); break;
+  }
+}
+
+// --- a warp's pipeline over the tiles of one field
+
+// What a lane does for the whole field: lane j issues the bulk copies of
+// stream j (contiguous input, and result) of full tiles.
+struct LaneStream {
+  const char* in;         // next tile's records, or nullptr
+  char* out;              // this tile's place in the result array, or nullptr
+  unsigned bytes;         // 32 records
+  unsigned slot, out_slot;
+};
+
+// index tile t (32 sites from 32 t) of every gathered stream, into ring place q
+__device__ __forceinline__ void fetch_indices(const BField& F, unsigned char* area, unsigned t, unsigned q, int nv,
+                                              int lane) {
+  if (lane >= nv) return;
+  for (int g = 0; g < F.ngather; g++) {
+    const BStream& S = F.s[F.gather[g]];
+    cp_async_4(area + S.idx_slot + q * 128u + (unsigned)lane * 4u, S.idx + (size_t)t * 32u + lane);
+  }
+}
+
+// records of tile t (nv sites) of every stream that a step reads (its index
+// tile has landed in ring place q): contiguous streams of a full tile by one
+// bulk copy each, lane j issuing stream j's; gathered H and D records by one
+// bulk copy per lane; gathered V and M records (24 and 72 B: no 16-B multiple
+// at 8-B steps) in 8-B pieces.  The stage's barrier gets one arrival with the
+// bytes to come.
+__device__ __forceinline__ void fetch_tile(const BField& F, LaneStream& L, unsigned char* area, unsigned char* stage,
+                                           uint64_t* bar, unsigned t, unsigned q, int nv, unsigned nw, int lane,
+                                           unsigned* err) {
+  unsigned tx = 0;
+  if (F.bulk && nv == 32) {
+    tx = F.tx;
+    if (L.in) {
+      bulk_g2s(stage + L.slot, L.in, L.bytes, bar, policy_evict_first());
+      L.in += (size_t)nw * L.bytes;
+    }
+  } else {
+    for (int j = 0; j < F.nstreams; j++) {
+      const BStream& S = F.s[j];
+      const unsigned rb = rec_b(S.kind);
+      if (S.used && !S.idx) run_in(stage + S.slot, S.base + (size_t)t * 32u * rb, (unsigned)nv * rb, lane);
     }
   }
-}
-
-template <int MC>
-__device__ __forceinline__ void exec_step(const BStep& S, const Rec<MC>& xa, const Rec<MC>& xb, Rec<MC>& y) {
-  const bool load = (S.eqop == PEQ || S.eqop == MEQ);
-  switch (S.op) {
-    case BOP_LMULT:
-      switch (S.kind_b * 4 + S.adja * 2 + S.adjb) {
-        case BK_V * 4 + 0: lmult_site<float, 3, 1, false, false>(S.eqop, load, xa, xb, y); break;
-        case BK_V * 4 + 2: lmult_site<float, 3, 1, true, false>(S.eqop, load, xa, xb, y); break;
-        case BK_H * 4 + 0: lmult_site<float, 3, 2, false, false>(S.eqop, load, xa, xb, y); break;
-        case BK_H * 4 + 2: lmult_site<float, 3, 2, true, false>(S.eqop, load, xa, xb, y); break;
-        case BK_M * 4 + 0: lmult_site<float, 3, 3, false, false>(S.eqop, load, xa, xb, y); break;
-        case BK_M * 4 + 1: lmult_site<float, 3, 3, false, true>(S.eqop, load, xa, xb, y); break;
-        case BK_M * 4 + 2: lmult_site<float, 3, 3, true, false>(S.eqop, load, xa, xb, y); break;
-        case BK_M * 4 + 3: lmult_site<float, 3, 3, true, true>(S.eqop, load, xa, xb, y); break;
-        default:
-          if constexpr (MC >= 12) {
-            if (S.adja)
-              lmult_site<float, 3, 4, true, false>(S.eqop, load, xa, xb, y);
-            else
-              lmult_site<float, 3, 4, false, false>(S.eqop, load, xa, xb, y);
-          }
-          break;
+  for (int g = 0; g < F.ngather; g++) {
+    const BStream& S = F.s[F.gather[g]];
+    const int* idx = reinterpret_cast<const int*>(area + S.idx_slot + q * 128u);
+    const int k = lane < nv ? idx[lane] : 0;
+    const bool ok = S.lim == 0u || (unsigned)k < S.lim || lane >= nv;
+    const unsigned bad = ~__ballot_sync(0xffffffffu, ok);
+    if (!ok) raise_dev_error(err, QLA_DEVERR_BAD_INDEX);
+    unsigned char* dst = stage + S.slot;
+    if (S.wide && (S.kind == BK_D || S.kind == BK_H)) {
+      const unsigned rb = rec_b(S.kind);
+      if (lane < nv) {
+        if (ok) {
+          bulk_g2s(dst + lane * rb, S.base + (long long)k * (int)rb, rb, bar, policy_evict_normal());
+        } else {
+          for (unsigned o = 0; o < rb; o += 16u) *reinterpret_cast<uint4*>(dst + lane * rb + o) = make_uint4(0, 0, 0, 0);
+        }
       }
-      break;
-    case BOP_SPPROJ:
-      if constexpr (MC >= 12) mu_sign_dispatch<SpprojOp<float, 3>::Body>(S.mu, S.sign, S.eqop, xa, y);
-      break;
-    case BOP_SPRECON:
-      if constexpr (MC >= 12) mu_sign_dispatch<SpreconOp<float, 3>::Body>(S.mu, S.sign, S.eqop, xa, y);
-      break;
-    case BOP_RTIMES:
-      switch (S.kind_r) {
-        case BK_V: rtimes_n<3>(S.eqop, S.r, xa, y); break;
-        case BK_H: rtimes_n<6>(S.eqop, S.r, xa, y); break;
-        case BK_M: rtimes_n<9>(S.eqop, S.r, xa, y); break;
-        default:
-          if constexpr (MC >= 12) rtimes_n<12>(S.eqop, S.r, xa, y);
-          break;
-      }
-      break;
-    default:
-      switch (S.kind_r) {
-        case BK_V: copy_n<3>(S.eqop, xa, y); break;
-        case BK_H: copy_n<6>(S.eqop, xa, y); break;
-        case BK_M: copy_n<9>(S.eqop, xa, y); break;
-        default:
-          if constexpr (MC >= 12) copy_n<12>(S.eqop, xa, y);
-          break;
-      }
-      break;
-  }
-}
-
-// stored result y of stream S: into the warp's output slice (out != nullptr,
-// lane `lane`) or straight to global memory (site i)
-template <int MC>
-__device__ __forceinline__ void put(const BStream& S, const Rec<MC>& y, unsigned char* out, int lane, long long i) {
-  switch (S.kind) {
-    case BK_V:
-      if (out) st_smem<3>(out + S.out_off + (unsigned)lane * 24u, y); else st_global<3>(S.base + i * 24, y);
-      break;
-    case BK_H:
-      if (out) st_smem<6>(out + S.out_off + (unsigned)lane * 48u, y); else st_global<6>(S.base + i * 48, y);
-      break;
-    case BK_M:
-      if (out) st_smem<9>(out + S.out_off + (unsigned)lane * 72u, y); else st_global<9>(S.base + i * 72, y);
-      break;
-    default:
-      if constexpr (MC >= 12) {
-        if (out) st_smem<12>(out + S.out_off + (unsigned)lane * 96u, y); else st_global<12>(S.base + i * 96, y);
-      }
-      break;
-  }
-}
-
-// One site through the field's whole program (the generic interpreter).
-template <int MC>
-__device__ __forceinline__ void run_program_generic(const BField& F, const SiteSrc& src, unsigned char* out,
-                                                    int lane) {
-  const int ns = F.nsteps;
-  Rec<MC> prev;
-  int prev_reg = -1;
-  for (int k = 0; k < ns; k++) {
-    const BStep S = F.st[k];  // uniform across the warp
-    Rec<MC> xa, xb, y;
-    fetch(xa, S.a, S.kind_a, F, src, prev, prev_reg);
-    if (S.op == BOP_LMULT) fetch(xb, S.b, S.kind_b, F, src, prev, prev_reg);
-    if (S.eqop == PEQ || S.eqop == MEQ)
-      fetch(y, S.load_stream >= 0 ? S.load_stream : S.dst, S.kind_r, F, src, prev, prev_reg);
-    exec_step(S, xa, xb, y);
-    if (S.spill) set_reg(src, S.dst - kReg0, S.kind_r, y);  // a later, non-adjacent step reads it
-    if (S.store >= 0) put(F.s[S.store], y, out, lane, src.i);
-    copy_rec(prev, y);
-    prev_reg = S.dst;
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Compiled program shapes.  A shape fixes each step's operation, operand
-// kinds and adjoints at compile time; a plan whose fields all share one
-// shape of the catalogue below runs a kernel instantiated for it: the steps
-// are unrolled, every record has its exact length and no step is decoded.
-// Operand streams and registers, eqops, mu / sign and the scalar stay
-// run-time values of the field's descriptor, and the per-site arithmetic is
-// the same as the interpreter's (bit-identical results).
-// where a step's operand comes from (classified by the planner)
-enum SrcKind : int { SRC_CONTIG = 0, SRC_GATHER = 1, SRC_INOUT = 2, SRC_PREV = 3, SRC_REG = 4, SRC_NONE = 5 };
-template <int OP, int KA, int KB, int ADJA, int ADJB, int SA, int SB, int EQOP = -1>  // EQOP -1: run time
-struct StepShape {
-  static constexpr int op = OP, ka = KA, kb = KB, adja = ADJA, adjb = ADJB, sa = SA, sb = SB, eqop = EQOP;
-  static constexpr int kr = OP == BOP_LMULT ? KB : OP == BOP_SPPROJ ? BK_H : OP == BOP_SPRECON ? BK_D : KA;
-};
-template <class... S>
-struct Shape {
-  static constexpr int nsteps = sizeof...(S);
-};
-struct GenericShape {};
-
-// The operand of a compiled shape's first step that is gathered (1: a, 2: b,
-// 0: none) and its record length in complex numbers.
-template <class SH>
-struct LeadGather {
-  static constexpr int which = 0, n = 0;
-};
-template <class S0, class... R>
-struct LeadGather<Shape<S0, R...>> {
-  static constexpr int which = S0::sb == SRC_GATHER ? 2 : S0::sa == SRC_GATHER ? 1 : 0;
-  static constexpr int n = which == 2 ? kncplx(S0::kb) : which == 1 ? kncplx(S0::ka) : 0;
-};
-
-// r = u * u2[nbr], w = r * v                          (config 4)
-using ShapeConfig4 = Shape<StepShape<BOP_LMULT, BK_M, BK_M, 0, 0, SRC_CONTIG, SRC_GATHER, EQ>,
-                           StepShape<BOP_LMULT, BK_M, BK_V, 0, 0, SRC_PREV, SRC_CONTIG, EQ>>;
-// out (eqop) sprecon(U spproj(D[nbr]))                 (one Wilson hop direction)
-using ShapeHop = Shape<StepShape<BOP_SPPROJ, BK_D, BK_D, 0, 0, SRC_GATHER, SRC_NONE>,
-                       StepShape<BOP_LMULT, BK_M, BK_H, 0, 0, SRC_CONTIG, SRC_PREV>,
-                       StepShape<BOP_SPRECON, BK_H, BK_H, 0, 0, SRC_PREV, SRC_NONE>>;
-// y (eqop) r x, w = U^+ y
-using ShapeAxpyMaD = Shape<StepShape<BOP_RTIMES, BK_D, BK_D, 0, 0, SRC_CONTIG, SRC_NONE>,
-                           StepShape<BOP_LMULT, BK_M, BK_D, 1, 0, SRC_CONTIG, SRC_PREV>>;
-// R = U U2^+, Q (eqop) R
-using ShapeMMaCopy = Shape<StepShape<BOP_LMULT, BK_M, BK_M, 0, 1, SRC_CONTIG, SRC_CONTIG>,
-                           StepShape<BOP_COPY, BK_M, BK_M, 0, 0, SRC_PREV, SRC_NONE>>;
-enum ShapeId : int { SH_GENERIC = 0, SH_CONFIG4 = 1, SH_HOP = 2, SH_AXPY_MAD = 3, SH_MMA_COPY = 4, SH_MULTI = 5 };
-
-template <class SS, int MC>
-__device__ __forceinline__ void exec_shaped(const BStep& S, const Rec<MC>& xa, const Rec<MC>& xb, Rec<MC>& y) {
-  const bool load = (S.eqop == PEQ || S.eqop == MEQ);
-  constexpr int NR = kncplx(SS::kr);
-  if constexpr (SS::op == BOP_LMULT) {
-    constexpr int NCOL = SS::kb == BK_V ? 1 : SS::kb == BK_H ? 2 : SS::kb == BK_D ? 4 : 3;
-    lmult_site<float, 3, NCOL, SS::adja != 0, SS::adjb != 0>(S.eqop, load, xa, xb, y);
-  } else if constexpr (SS::op == BOP_SPPROJ) {
-    mu_sign_dispatch<SpprojOp<float, 3>::Body>(S.mu, S.sign, S.eqop, xa, y);
-  } else if constexpr (SS::op == BOP_SPRECON) {
-    mu_sign_dispatch<SpreconOp<float, 3>::Body>(S.mu, S.sign, S.eqop, xa, y);
-  } else if constexpr (SS::op == BOP_RTIMES) {
-    rtimes_n<NR>(S.eqop, S.r, xa, y);
-  } else {
-    copy_n<NR>(S.eqop, xa, y);
-  }
-}
-
-template <int N, int MC>
-__device__ __forceinline__ void put_n(const BStream& S, const Rec<MC>& y, unsigned char* out, int lane, long long i) {
-  if (out)
-    st_smem<N>(out + S.out_off + (unsigned)lane * (N * 8), y);
-  else
-    st_global<N>(S.base + i * (N * 8), y);
-}
-
-// operand `ref` of compile-time source SRC and length N
-template <int SRC, int N, int MC>
-__device__ __forceinline__ void fetch_src(Rec<MC>& x, int ref, const BField& F, const SiteSrc& src,
-                                          const Rec<MC>& prev) {
-  if constexpr (SRC == SRC_PREV) {
-    copy_rec_n<N>(x, prev);
-  } else if constexpr (SRC == SRC_REG) {
-    reg_load<N>(x, src, ref - kReg0);
-  } else if constexpr (SRC == SRC_GATHER) {
-    const BStream& S = F.s[ref];
-    long long j = src.stage ? reinterpret_cast<const int*>(src.stage + S.stage_off)[src.t] : S.idx[src.i];
-    if (S.nsrc > 0 && (j < 0 || j >= S.nsrc)) {
-      raise_dev_error(src.err, QLA_DEVERR_BAD_INDEX);
-      zero_rec(x);
+      tx += rb * (unsigned)(nv - __popc(bad));
     } else {
-      ld_global<N>(x, S.base + j * (long long)(N * 8));
+      switch (S.kind) {
+        case BK_V: gather_pieces<3>(dst, S.base, idx, nv, bad, lane); break;
+        case BK_H: gather_pieces<6>(dst, S.base, idx, nv, bad, lane); break;
+        case BK_D: gather_pieces<12>(dst, S.base, idx, nv, bad, lane); break;
+        default: gather_pieces<9>(dst, S.base, idx, nv, bad, lane); break;
+      }
     }
-  } else {  // SRC_CONTIG, SRC_INOUT
-    const BStream& S = F.s[ref];
-    if (src.stage)
-      ld_smem<N>(x, src.stage + S.stage_off + (unsigned)src.t * (N * 8));
-    else if constexpr (SRC == SRC_INOUT)
-      ld_global_rw<N>(x, S.base + src.i * (N * 8));
+  }
+  if (lane == 0) {
+    if (tx)
+      mbar_arrive_expect_tx(bar, tx);
     else
-      ld_global<N>(x, S.base + src.i * (N * 8));
+      mbar_arrive(bar);
   }
 }
 
-template <int MC, int K, class SS, class... Rest>
-__device__ __forceinline__ void run_shaped(const BField& F, const SiteSrc& src, unsigned char* out, int lane,
-                                           Rec<MC>& prev, int prev_reg) {
-  BStep S = F.st[K];
-  if constexpr (SS::eqop >= 0) S.eqop = SS::eqop;  // a compiled eqop (the planner matched it)
-  constexpr int NA = kncplx(SS::ka), NB = kncplx(SS::kb), NR = kncplx(SS::kr);
-  Rec<MC> xa, xb, y;
-  fetch_src<SS::sa, NA>(xa, S.a, F, src, prev);
-  if constexpr (SS::op == BOP_LMULT) fetch_src<SS::sb, NB>(xb, S.b, F, src, prev);
-  if (S.eqop == PEQ || S.eqop == MEQ) fetch_n<NR>(y, S.load_stream >= 0 ? S.load_stream : S.dst, F, src, prev, prev_reg);
-  exec_shaped<SS>(S, xa, xb, y);
-  if (S.spill) reg_store<NR>(src, S.dst - kReg0, y);
-  if (S.store >= 0) put_n<NR>(F.s[S.store], y, out, lane, src.i);
-  if constexpr (sizeof...(Rest) > 0) {
-    copy_rec_n<NR>(prev, y);
-    run_shaped<MC, K + 1, Rest...>(F, src, out, lane, prev, S.dst);
-  }
-}
-template <int MC, class... SS>
-__device__ __forceinline__ void run_shape(Shape<SS...>, const BField& F, const SiteSrc& src, unsigned char* out,
-                                          int lane) {
-  Rec<MC> prev;
-  run_shaped<MC, 0, SS...>(F, src, out, lane, prev, -1);
-}
-
-// A plan whose fields all have catalogue shapes, but not one shape, runs the
-// multi-shape kernel: each field's compiled path, chosen per tile (uniform).
-// Other plans run the interpreter.
-struct MultiShape {};
-template <int MC, class SH>
-__device__ __forceinline__ void run_program(const BField& F, const SiteSrc& src, unsigned char* out, int lane) {
-  if constexpr (std::is_same<SH, GenericShape>::value) {
-    run_program_generic<MC>(F, src, out, lane);
-  } else if constexpr (std::is_same<SH, MultiShape>::value) {
-    switch (F.shape) {
-      case SH_CONFIG4: run_shape<MC>(ShapeConfig4{}, F, src, out, lane); break;
-      case SH_MMA_COPY: run_shape<MC>(ShapeMMaCopy{}, F, src, out, lane); break;
-      case SH_HOP:
-        if constexpr (MC >= 12) run_shape<MC>(ShapeHop{}, F, src, out, lane);
-        break;
-      default:
-        if constexpr (MC >= 12) run_shape<MC>(ShapeAxpyMaD{}, F, src, out, lane);
-        break;
-    }
-  } else {
-    run_shape<MC>(SH{}, F, src, out, lane);
-  }
-}
-
-// Copy of field f's descriptor in this warp's shared slot (all lanes take
-// part; the caller's lanes then read it from shared memory, not global), kept
-// while consecutive tiles belong to the same field.
-constexpr int kDescWords = (int)((sizeof(BField) + 15) / 16);  // 16-B words
-__device__ __forceinline__ const BField& cached_field(const BatchParams& p, int f, int& cached, uint4* slot,
-                                                      int lane) {
-  if (f != cached) {
-    __syncwarp();  // every lane is done with the previous field's descriptor
-    const uint4* src = reinterpret_cast<const uint4*>(p.fields + f);
-    for (int w = lane; w < kDescWords; w += 32) slot[w] = __ldg(src + w);
-    __syncwarp();
-    cached = f;
-  }
-  return *reinterpret_cast<const BField*>(slot);
-}
-// the same for the producer, a single lane
-__device__ __forceinline__ const BField& cached_field_1(const BatchParams& p, int f, int& cached, uint4* slot) {
-  if (f != cached) {
-    const uint4* src = reinterpret_cast<const uint4*>(p.fields + f);
-    for (int w = 0; w < kDescWords; w++) slot[w] = __ldg(src + w);
-    cached = f;
-  }
-  return *reinterpret_cast<const BField*>(slot);
-}
-
-// Dynamic smem: [full[8], empty[8] | abort | tile0 table (8 KB) | S stages |
-//               NW output slices | step registers (only when some
-//               program spills one): 2 x 12 complex x T | (NW + 1) field
-//               descriptors]
-// 128 consumer threads (or 64) and one producer warp.  Blocks per SM (the
-// register budget each instance compiles to without spilling): a compiled
-// shape four (V / H / M records, <= 96 registers) or three (DiracFermions,
-// <= 128); the interpreter and the multi-shape kernel three (V / H / M) or
-// two (DiracFermions).
-constexpr int kBatchThreadsMax = 160;
-template <int MC, class SH>
-constexpr int batch_min_blocks() {
-  constexpr bool compiled = !std::is_same<SH, GenericShape>::value && !std::is_same<SH, MultiShape>::value;
-  // (the multi-shape kernel at 12 complex numbers: three blocks with spills
-  // measured 0.39 of HBM on a config-4 / hop mix, two 0.38, one at 254
-  // registers 0.32)
-  constexpr bool multi = std::is_same<SH, MultiShape>::value;
-  return MC == 9 ? (compiled ? 4 : 3) : (compiled || multi ? 3 : 2);
-}
-template <int MC, class SH>
-__global__ void __launch_bounds__(kBatchThreadsMax, batch_min_blocks<MC, SH>()) batch_program_kernel(
-    const BatchParams p) {
+// A warp's shared memory: [two stage barriers | field descriptor | index
+// tiles (fixed_bytes) | one or two stages].
+__global__ void __launch_bounds__(128, 4) batch_program_kernel(const BatchParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
-  const int S = p.stages;
-  const int NW = (blockDim.x >> 5) - 1;
-  const int T = NW * 32;
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem);
-  uint64_t* empty = full + 8;
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + 128);
-  long long* tile0 = reinterpret_cast<long long*>(smem + 256);
-  unsigned char* stages = smem + 256 + 8 * kMaxFields;
-  unsigned char* outbuf = stages + (size_t)S * p.stage_bytes;
-  unsigned char* regs = outbuf + (size_t)NW * p.out_slice_bytes;  // 2 x 12 complex per thread, if needed
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // Tiles are dealt to the blocks in groups of p.chunk consecutive tiles,
-  // round-robin: consecutive tiles of a block then mostly belong to one
-  // field, so that a warp seldom reloads its cached field descriptor (tiles
-  // dealt one by one land in a new field nearly every time on small fields).
-  // Block b's k-th tile is tile_of(k).
-  const long long C = p.chunk, ngroups = (p.ntiles + C - 1) / C;
-  long long my = 0;
-  if ((long long)blockIdx.x < ngroups) {
-    const long long mg = (ngroups - 1 - (long long)blockIdx.x) / gridDim.x + 1;  // groups of this block
-    const bool owns_last = (ngroups - 1 - (long long)blockIdx.x) % gridDim.x == 0;
-    my = mg * C - (owns_last ? ngroups * C - p.ntiles : 0);
-  }
-  auto tile_of = [&](long long k) { return ((long long)blockIdx.x + (k / C) * gridDim.x) * C + k % C; };
-  uint4* desc = reinterpret_cast<uint4*>(regs + (p.spill_regs ? (size_t)2 * 12 * 8 * T : 0)) + (size_t)warp * kDescWords;
-  int cached = -1;
-
-  for (int f = tid; f < p.nfields; f += blockDim.x) tile0[f] = p.fields[f].tile0;
-  if (tid == 0) {
-    for (int s = 0; s < S; s++) {
-      mbar_init(&full[s], 1);
-      mbar_init(&empty[s], (unsigned)NW);
-    }
-    *abort_flag = 0;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned nw = blockDim.x >> 5;
+  unsigned char* mine = smem + (size_t)warp * p.warp_bytes;
+  uint64_t* bar = reinterpret_cast<uint64_t*>(mine);
+  uint4* desc = reinterpret_cast<uint4*>(mine + 16);
+  unsigned char* area = reinterpret_cast<unsigned char*>(desc + kDescWords);
+  unsigned char* stages = area + p.fixed_bytes;
+  const BField& F = *reinterpret_cast<const BField*>(desc);
+  if (lane == 0) {
+    mbar_init(&bar[0], 1);
+    mbar_init(&bar[1], 1);
     mbar_init_fence();
   }
-  __syncthreads();
-  long long issued = 0;
-
-  if (warp == NW) {
-    // ------------------------------------------------------------ producer
-    if (lane == 0) {
-      const uint64_t pol = policy_evict_first();
-      long long k = 0, round = 0;
-      int s = 0;
-      for (; k < my; k++) {
-        if (round > 0 && !mbar_wait_bounded(&empty[s], (uint32_t)((round - 1) & 1), p.err, 2000000000ull,
-                                            abort_flag)) {
-          *abort_flag = 1;
-          break;
-        }
-        const long long g = tile_of(k);
-        const BField& F = cached_field_1(p, field_of(tile0, p.nfields, g, cached), cached, desc);
-        const long long site0 = (g - F.tile0) * T;
-        unsigned char* st = stages + (size_t)s * p.stage_bytes;
-        if (!F.direct && site0 + T <= F.n) {
-          mbar_arrive_expect_tx(&full[s], F.tx_bytes);
-          for (int j = 0; j < F.nstreams; j++) {
-            const BStream& B = F.s[j];
-            const unsigned rb = (unsigned)kncplx(B.kind) * 8u;
-            if (B.role == BR_IN && B.idx)
-              bulk_g2s(st + B.stage_off, B.idx + site0, (unsigned)T * 4u, &full[s], pol);
-            else if (B.role != BR_OUT)
-              bulk_g2s(st + B.stage_off, B.base + site0 * rb, (unsigned)T * rb, &full[s], pol);
-          }
-        } else {
-          mbar_arrive(&full[s]);  // partial / unaligned tile: consumers use plain loads
-        }
-        if (++s == S) {
-          s = 0;
-          round++;
-        }
+  unsigned cnt = 0;  // tiles fetched: stage cnt & 1, parity (cnt >> 1) & 1
+  bool alive = true;
+  for (int run = blockIdx.x; run < p.runs && alive; run += gridDim.x) {
+    // a run's tiles are dealt to the block's warps one by one
+    long long g = p.start[run] + warp;
+    const long long gend = p.start[run + 1];
+    if (g >= gend) continue;
+    int f;
+    {
+      int lo = 0, hi = p.nfields - 1;  // last field with tile0 <= g
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (p.fields[mid].tile0 <= g)
+          lo = mid;
+        else
+          hi = mid - 1;
       }
-      issued = k;
+      f = lo;
     }
-  } else {
-    // ------------------------------------------------------------ consumers
-    const uint64_t pol = policy_evict_first();
-    unsigned char* myout = outbuf + (size_t)warp * p.out_slice_bytes;
-    int s = 0;
-    uint32_t par = 0;
-    for (long long k = 0; k < my; k++) {
-      if (!mbar_wait_bounded(&full[s], par, p.err, 2000000000ull, abort_flag)) {
-        *abort_flag = 1;
-        break;
-      }
-      const long long g = tile_of(k);
-      const BField& F = cached_field(p, field_of(tile0, p.nfields, g, cached), cached, desc, lane);
-      const long long site0 = (g - F.tile0) * T;
-      const int t = warp * 32 + lane;
-      const long long i = site0 + t;
-      // staged: a full tile of a 16-B aligned field, in the stage; else the
-      // same program with plain loads and stores (partial / unaligned tiles)
-      const bool staged = !F.direct && site0 + T <= F.n;
-      // a compiled shape that starts with a gather: when the block's next tile
-      // is the next tile of this field, load this lane's index of it now and
-      // prefetch its gathered record into L2 after this tile's arithmetic
-      int pf_j = -1;
-      if constexpr (LeadGather<SH>::which != 0) {
-        if (k + 1 < my && tile_of(k + 1) == g + 1 && i + T < F.n) {
-          const BStream& G = F.s[LeadGather<SH>::which == 2 ? F.st[0].b : F.st[0].a];
-          pf_j = __ldg(G.idx + i + T);
+    for (; g < gend && alive; f++) {
+      const uint4* src = reinterpret_cast<const uint4*>(p.fields + f);
+      for (int k = lane; k < kDescWords; k += 32) desc[k] = __ldg(src + k);
+      __syncwarp();
+      const long long ntf = (F.n + 31) / 32;  // tiles of this field (an empty field has none)
+      const int ntail = (int)(F.n & 31);      // sites of a partial last tile
+      unsigned t = (unsigned)(g - F.tile0 < ntf ? g - F.tile0 : ntf);  // (a warp may skip a small field)
+      const unsigned tend = (unsigned)(gend - F.tile0 < ntf ? gend - F.tile0 : ntf);
+      auto sites = [&](unsigned u) { return (ntail && (long long)u + 1 == ntf) ? ntail : 32; };
+      if (g < F.tile0 + tend) g += ((F.tile0 + tend - g + nw - 1) / nw) * nw;  // this warp's first tile behind it
+      if (t < tend) {
+        LaneStream L{nullptr, nullptr, 0u, 0u, 0u};
+        if (lane < F.nstreams) {
+          const BStream& S = F.s[lane];
+          L.bytes = 32u * rec_b(S.kind);
+          L.slot = S.slot;
+          L.out_slot = S.out;
+          char* at = S.base + (size_t)t * L.bytes;
+          if (S.used && !S.idx) L.in = at;
+          if (S.role != BR_IN) L.out = at;
         }
-      }
-      unsigned char* ob = myout;
-      if (staged) {
-        if (lane == 0) bulk_wait_read<0>();  // the slice is no longer read by this warp's previous store
+        // fill the pipeline: indices of two tiles, records of the first
+        unsigned q = 0;  // ring place of tile t's indices
+        fetch_indices(F, area, t, 0, sites(t), lane);
+        cp_async_wait_all();
         __syncwarp();
-      } else {
-        release_stage(&empty[s], lane);  // this warp is done with the stage
-      }
-      if (staged || i < F.n)  // one call site: the program is inlined once
-        run_program<MC, SH>(F, SiteSrc{staged ? stages + (size_t)s * p.stage_bytes : nullptr, t, i, p.err, regs, T},
-                            staged ? ob : nullptr, lane);
-      if constexpr (LeadGather<SH>::which != 0) {
-        const BStream& G = F.s[LeadGather<SH>::which == 2 ? F.st[0].b : F.st[0].a];
-        if (pf_j >= 0 && (G.nsrc <= 0 || pf_j < G.nsrc)) {  // only an index the gather would dereference
-          constexpr long long RBG = LeadGather<SH>::n * 8;
-          const char* q = G.base + (long long)pf_j * RBG;
-          prefetch_l2(q);
-          prefetch_l2(q + RBG - 8);
-        }
-      }
-      if (staged) {
-        // every lane orders its reads of the stage and its writes of the
-        // slice before the async proxy: the slice's bulk stores below, and
-        // the producer's next bulk copy into the stage released here
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(&empty[s]);  // this warp is done with the stage
-          const long long s0 = site0 + warp * 32;
-          for (int j = 0; j < F.nstreams; j++) {
-            const BStream& B = F.s[j];
-            if (B.role == BR_IN) continue;
-            const unsigned rb = (unsigned)kncplx(B.kind) * 8u;
-            bulk_s2g(B.base + s0 * rb, ob + B.out_off, 32u * rb, pol);
+        // stage and barrier of the c-th tile this warp fetches, and its parity
+        auto place = [&](unsigned c) { return p.stages == 2 ? c & 1u : 0u; };
+        auto parity = [&](unsigned c) { return (p.stages == 2 ? c >> 1 : c) & 1u; };
+        fetch_tile(F, L, area, stages + place(cnt) * p.stage_bytes, &bar[place(cnt)], t, 0, sites(t), nw, lane, p.err);
+        if (t + nw < tend) fetch_indices(F, area, t + nw, 1, sites(t + nw), lane);
+        for (; t < tend; t += nw, cnt++) {
+          cp_async_wait_all();
+          bulk_wait_read<0>();  // the previous tile's results have left their slots
+          if (!mbar_wait_bounded(&bar[place(cnt)], parity(cnt), p.err)) alive = false;
+          alive = __all_sync(0xffffffffu, alive);  // this tile's records and the next tile's indices have landed
+          if (!alive) break;
+          const unsigned q1 = q == 2u ? 0u : q + 1u, q2 = q1 == 2u ? 0u : q1 + 1u;
+          unsigned char* stage = stages + place(cnt) * p.stage_bytes;
+          if (p.stages == 2 && t + nw < tend)
+            fetch_tile(F, L, area, stages + (~cnt & 1u) * p.stage_bytes, &bar[~cnt & 1u], t + nw, q1, sites(t + nw), nw,
+                       lane, p.err);
+          if (t + 2 * nw < tend) fetch_indices(F, area, t + 2 * nw, q2, sites(t + 2 * nw), lane);
+          q = q1;
+          const int nv = sites(t);
+          // (the lanes behind a partial tile compute on what lies in their slots;
+          // nothing of it is stored)
+          const Slots sl{stage, lane};
+          for (int k = 0; k < F.nsteps; k++) run_step(F.st[k], sl);
+          // orders this lane's reads and writes of the slots before the async
+          // proxy: the bulk stores below and the next bulk copies into the stage
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (F.bulk && nv == 32) {
+            if (L.out) {
+              bulk_s2g(L.out, stage + L.out_slot, L.bytes,
+                       policy_evict_first());
+              bulk_commit();
+              L.out += (size_t)nw * L.bytes;
+            }
+          } else {
+            for (int j = 0; j < F.nstreams; j++) {
+              const BStream& S = F.s[j];
+              const unsigned rb = rec_b(S.kind);
+              if (S.role != BR_IN)
+                run_out(S.base + (size_t)t * 32u * rb, stage + S.out,
+                        (unsigned)nv * rb, lane);
+            }
+            __syncwarp();  // the result slots are free
           }
-          bulk_commit();
+          if (p.stages == 1 && t + nw < tend) {
+            bulk_wait_read<0>();
+            __syncwarp();
+            fetch_tile(F, L, area, stages, bar, t + nw, q, sites(t + nw), nw, lane, p.err);
+          }
         }
-      } else if (lane == 0) {
-        bulk_commit();  // an empty group keeps the slice bookkeeping aligned
       }
-      if (++s == S) {
-        s = 0;
-        par ^= 1u;
-      }
+      __syncwarp();  // every lane is done with this field's descriptor
     }
-    if (lane == 0) bulk_wait_all<0>();
   }
-  __syncthreads();
-  if (*abort_flag && warp == NW && lane == 0) {
-    // a wait failed: wait (bounded) for every load still in flight before the
-    // block's shared memory is released
-    for (long long kk = (issued > S ? issued - S : 0); kk < issued; kk++)
-      if (!mbar_wait_bounded(&full[kk % S], (uint32_t)((kk / S) & 1), p.err, 200000000ull, nullptr))
+  // a wait that gave up: wait (bounded) once more for the copies of both
+  // stages before the warp's shared memory can be released
+  if (!alive) {
+    for (int s = 0; s < p.stages; s++)
+      if (!mbar_wait_bounded(&bar[p.stages == 2 ? (cnt + s) & 1u : 0u], (p.stages == 2 ? (cnt + s) >> 1 : cnt) & 1u,
+                             p.err, 200000000ull) &&
+          lane == 0)
         raise_dev_error(p.err, QLA_DEVERR_BULK_TIMEOUT);
+    cp_async_wait_all();
   }
+  bulk_wait_all<0>();
 }
 
 // ---------------------------------------------------------------------------
@@ -781,19 +498,17 @@ static bool plan_error(const char* who, int f, int k, const char* what) {
 
 static bool aligned(const void* p, unsigned a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
 
-// Checks one program and fills its device descriptor (kinds, stage offsets
-// for a tile of T sites, output slice offsets).  Returns false with the
-// sticky error set when the program is malformed.
-static bool build_field(const char* who, int f, const qlagpu_F3_batch_program& q, int T, BField& b,
-                        unsigned& stage_bytes, unsigned& out_slice_bytes, bool& spills, bool& uses_d) {
+// Checks one program and fills its device descriptor: kinds, step codes and
+// the shared-memory slots of everything the steps read and make.  Returns
+// false with the sticky error set when the program is malformed.
+static bool build_field(const char* who, int f, const qlagpu_F3_batch_program& q, BField& b, unsigned& fixed_bytes,
+                        unsigned& stage_bytes, long long& cost) {
   std::memset(&b, 0, sizeof(b));
   if (q.n < 0 || q.nstreams < 0 || q.nstreams > kMaxStreams || q.nsteps < 1 || q.nsteps > kMaxSteps)
     return plan_error(who, f, -1, "need n >= 0, 0..8 streams and 1..8 steps");
   b.nstreams = q.nstreams;
   b.nsteps = q.nsteps;
   b.n = q.n;
-  bool al16 = true;
-  unsigned off = 0, oo = 0;
   for (int j = 0; j < q.nstreams; j++) {
     const qlagpu_batch_stream& s = q.stream[j];
     BStream& d = b.s[j];
@@ -806,29 +521,15 @@ static bool build_field(const char* who, int f, const qlagpu_F3_batch_program& q
       return plan_error(who, f, -1, "stream base must be 8-B aligned and an index 4-B aligned");
     d.base = static_cast<char*>(s.base);
     d.idx = s.index;
-    d.nsrc = s.index ? s.nsrc : 0;
+    d.lim = s.index ? (unsigned)(s.nsrc < 0x7fffffffLL ? s.nsrc : 0x80000000LL) : 0u;
     d.kind = s.kind;
     d.role = s.role;
-    const unsigned rb = (unsigned)kncplx(s.kind) * 8u;
-    if (s.role == BR_IN && s.index) {
-      d.stage_off = off;
-      off += ((unsigned)T * 4u + 15u) & ~15u;
-      b.tx_bytes += (unsigned)T * 4u;
-      al16 = al16 && aligned(s.index, 16);
-    } else if (s.role != BR_OUT) {
-      d.stage_off = off;
-      off += ((unsigned)T * rb + 15u) & ~15u;
-      b.tx_bytes += (unsigned)T * rb;
-    }
-    if (!s.index || s.role != BR_IN) al16 = al16 && aligned(s.base, 16);
-    if (s.role != BR_IN) {
-      d.out_off = oo;
-      oo += 32u * rb;
-    }
+    d.wide = aligned(s.base, 16) ? 1 : 0;
   }
-  b.direct = al16 ? 0 : 1;
-  int regkind[2] = {-1, -1};
-  bool stored[kMaxStreams] = {false};
+  b.bulk = 1;
+  int regkind[2] = {-1, -1}, kind_a[kMaxSteps], kind_r[kMaxSteps], load_stream[kMaxSteps];
+  int store_step[kMaxStreams];
+  for (int j = 0; j < kMaxStreams; j++) store_step[j] = -1;
   auto opnd_kind = [&](int ref, int& kind) -> const char* {
     if (ref == kReg0 || ref == kReg1) {
       kind = regkind[ref - kReg0];
@@ -842,146 +543,152 @@ static bool build_field(const char* who, int f, const qlagpu_F3_batch_program& q
   for (int k = 0; k < q.nsteps; k++) {
     const qlagpu_batch_step& s = q.step[k];
     BStep& d = b.st[k];
-    d.op = s.op;
+    int kind_b = -1;
     d.eqop = s.eqop;
-    d.a = s.a;
-    d.b = s.b;
-    d.dst = s.dst;
-    d.store = s.store;
-    d.adja = s.adja ? 1 : 0;
-    d.adjb = s.adjb ? 1 : 0;
     d.mu = s.mu;
     d.sign = s.sign == 1 ? 1 : -1;
     d.r = s.r;
-    d.load_stream = -1;
+    load_stream[k] = -1;
     if (s.op < 0 || s.op > 4) return plan_error(who, f, k, "unknown op");
     if (s.eqop < 0 || s.eqop > 3) return plan_error(who, f, k, "eqop out of range");
     if (s.dst != kReg0 && s.dst != kReg1) return plan_error(who, f, k, "dst must be QLAGPU_REG0 or QLAGPU_REG1");
-    if (const char* e = opnd_kind(s.a, d.kind_a)) return plan_error(who, f, k, e);
+    if (const char* e = opnd_kind(s.a, kind_a[k])) return plan_error(who, f, k, e);
     switch (s.op) {
       case BOP_LMULT:
-        if (d.kind_a != BK_M) return plan_error(who, f, k, "LMULT: a must be a colour matrix");
-        if (const char* e = opnd_kind(s.b, d.kind_b)) return plan_error(who, f, k, e);
-        if (d.adjb && d.kind_b != BK_M) return plan_error(who, f, k, "LMULT: adjb needs a colour-matrix b");
-        d.kind_r = d.kind_b;
+        if (kind_a[k] != BK_M) return plan_error(who, f, k, "LMULT: a must be a colour matrix");
+        if (const char* e = opnd_kind(s.b, kind_b)) return plan_error(who, f, k, e);
+        if (s.adjb && kind_b != BK_M) return plan_error(who, f, k, "LMULT: adjb needs a colour-matrix b");
+        kind_r[k] = kind_b;
+        d.code = SC_LMULT + kind_b * 4 + (s.adja ? 2 : 0) + (s.adjb ? 1 : 0);
         break;
       case BOP_SPPROJ:
-        if (d.kind_a != BK_D) return plan_error(who, f, k, "SPPROJ: a must be a DiracFermion");
+        if (kind_a[k] != BK_D) return plan_error(who, f, k, "SPPROJ: a must be a DiracFermion");
         if (s.mu < 0 || s.mu > 4) return plan_error(who, f, k, "mu must be 0..4");
-        d.kind_r = BK_H;
+        kind_r[k] = BK_H;
+        d.code = SC_SPPROJ;
         break;
       case BOP_SPRECON:
-        if (d.kind_a != BK_H) return plan_error(who, f, k, "SPRECON: a must be a HalfFermion");
+        if (kind_a[k] != BK_H) return plan_error(who, f, k, "SPRECON: a must be a HalfFermion");
         if (s.mu < 0 || s.mu > 4) return plan_error(who, f, k, "mu must be 0..4");
-        d.kind_r = BK_D;
+        kind_r[k] = BK_D;
+        d.code = SC_SPRECON;
         break;
       default:
-        d.kind_r = d.kind_a;
+        kind_r[k] = kind_a[k];
+        d.code = (s.op == BOP_RTIMES ? SC_RTIMES : SC_COPY) + kind_r[k];
         break;
     }
-    if (s.op != BOP_LMULT) d.kind_b = d.kind_a;
     if (s.store >= 0) {
       if (s.store >= q.nstreams || q.stream[s.store].role == BR_IN)
         return plan_error(who, f, k, "store must name an OUT or INOUT stream");
-      if (q.stream[s.store].kind != d.kind_r) return plan_error(who, f, k, "stored stream has another kind");
-      if (stored[s.store]) return plan_error(who, f, k, "a stream is stored by more than one step");
-      stored[s.store] = true;
+      if (q.stream[s.store].kind != kind_r[k]) return plan_error(who, f, k, "stored stream has another kind");
+      if (store_step[s.store] >= 0) return plan_error(who, f, k, "a stream is stored by more than one step");
+      store_step[s.store] = k;
     } else if (s.store != -1) {
       return plan_error(who, f, k, "store must be a stream or -1");
     }
     if (s.eqop == PEQ || s.eqop == MEQ) {
       if (s.store >= 0 && q.stream[s.store].role == BR_INOUT) {
-        d.load_stream = s.store;
-      } else if (regkind[s.dst - kReg0] != d.kind_r) {
+        load_stream[k] = s.store;
+      } else if (regkind[s.dst - kReg0] != kind_r[k]) {
         return plan_error(who, f, k, "peq / meq needs an INOUT store stream or a dst register of the result kind");
       }
     }
-    regkind[s.dst - kReg0] = d.kind_r;
+    regkind[s.dst - kReg0] = kind_r[k];
   }
   for (int j = 0; j < q.nstreams; j++)
-    if (q.stream[j].role != BR_IN && !stored[j]) return plan_error(who, f, -1, "an output stream is never stored");
-  // register liveness: a register read by a step other than the one right
-  // after its writer is also kept in shared memory (the writer spills it)
+    if (q.stream[j].role != BR_IN && store_step[j] < 0)
+      return plan_error(who, f, -1, "an output stream is never stored");
+
+  // last step that reads each stream (-1: none)
+  int last_read[kMaxStreams];
+  for (int j = 0; j < kMaxStreams; j++) last_read[j] = -1;
   for (int k = 0; k < q.nsteps; k++) {
-    const BStep& d = b.st[k];
-    const int reads[3] = {d.a, d.op == BOP_LMULT ? d.b : -1,
-                          ((d.eqop == PEQ || d.eqop == MEQ) && d.load_stream < 0) ? d.dst : -1};
-    for (int r : reads) {
-      if (r != kReg0 && r != kReg1) continue;
-      int w = k - 1;
-      while (w >= 0 && b.st[w].dst != r) w--;
-      if (w >= 0 && w != k - 1) {
-        b.st[w].spill = 1;
-        spills = true;
+    const qlagpu_batch_step& s = q.step[k];
+    if (s.a < kMaxStreams) last_read[s.a] = k;
+    if (s.op == BOP_LMULT && s.b < kMaxStreams) last_read[s.b] = k;
+    if (load_stream[k] >= 0) last_read[load_stream[k]] = k;
+  }
+  // Places.  Every value a step reads or makes has a region of the stage: the
+  // streams' records from the start, a result from its step on.  A result
+  // takes the smallest region that fits of those whose value has been read
+  // for the last time (by this step at the latest), else a new one.  Values
+  // that are stored stay until the tile's end.
+  struct Region {
+    unsigned off, size;
+    int until;  // last step that reads its value; nsteps: stored at the end
+  };
+  std::vector<Region> regions;
+  unsigned fixed = 0, stage = 0;
+  // a tile's cost, in units of a site's bytes: 200 for the loop itself, 40 per
+  // step, a byte per byte, a half per floating-point operation (fitted to the
+  // times of five programs run alone, which it gives within 10 %)
+  cost = 200 + 40 * q.nsteps;
+  int stream_region[kMaxStreams], reg_region[2] = {-1, -1};
+  auto new_region = [&](unsigned size, int until) {
+    regions.push_back(Region{stage, size, until});
+    stage += size;
+    return (int)regions.size() - 1;
+  };
+  for (int j = 0; j < q.nstreams; j++) {
+    BStream& d = b.s[j];
+    stream_region[j] = -1;
+    d.used = last_read[j] >= 0;
+    if (d.used) {
+      stream_region[j] = new_region(32u * rec_b(d.kind), last_read[j]);
+      d.slot = regions[(size_t)stream_region[j]].off;
+      cost += rec_b(d.kind) + (d.idx ? 4u : 0u);
+      if (!d.idx) {
+        b.tx += 32u * rec_b(d.kind);
+        if (!d.wide) b.bulk = 0;
+      } else {
+        d.idx_slot = fixed;
+        fixed += 3u * 128u;
+        b.gather[b.ngather++] = j;
       }
     }
+    if (d.role == BR_IN) continue;
+    if (!d.wide) b.bulk = 0;
+    cost += rec_b(d.kind);
   }
-  // operand sources, for matching a compiled shape
+  // steps that read step k's result through its register, the last of them
+  auto last_use = [&](int k) {
+    const int r = q.step[k].dst;
+    int last = k;
+    for (int m = k + 1; m < q.nsteps; m++) {
+      const qlagpu_batch_step& s = q.step[m];
+      if (s.a == r || (s.op == BOP_LMULT && s.b == r) ||
+          ((s.eqop == PEQ || s.eqop == MEQ) && load_stream[m] < 0 && s.dst == r))
+        last = m;
+      if (s.dst == r) break;
+    }
+    return last;
+  };
   for (int k = 0; k < q.nsteps; k++) {
+    const qlagpu_batch_step& s = q.step[k];
     BStep& d = b.st[k];
-    auto src_of = [&](int ref) {
-      if (ref == kReg0 || ref == kReg1) return (k > 0 && b.st[k - 1].dst == ref) ? (int)SRC_PREV : (int)SRC_REG;
-      if (q.stream[ref].role == BR_INOUT) return (int)SRC_INOUT;
-      return q.stream[ref].index ? (int)SRC_GATHER : (int)SRC_CONTIG;
-    };
-    d.src_a = src_of(d.a);
-    d.src_b = d.op == BOP_LMULT ? src_of(d.b) : (int)SRC_NONE;
+    const int dr = s.dst - kReg0;
+    auto region_of = [&](int ref) { return ref >= kReg0 ? reg_region[ref - kReg0] : stream_region[ref]; };
+    d.a = regions[(size_t)region_of(s.a)].off;
+    if (s.op == BOP_LMULT) d.b = regions[(size_t)region_of(s.b)].off;
+    if (s.eqop == PEQ || s.eqop == MEQ)
+      d.old = regions[(size_t)(load_stream[k] >= 0 ? stream_region[load_stream[k]] : reg_region[dr])].off;
+    const unsigned need = 32u * rec_b(kind_r[k]);
+    int best = -1;
+    for (int m = 0; m < (int)regions.size(); m++)
+      if (regions[(size_t)m].until <= k && regions[(size_t)m].size >= need &&
+          (best < 0 || regions[(size_t)m].size < regions[(size_t)best].size))
+        best = m;
+    if (best < 0) best = new_region(need, 0);
+    regions[(size_t)best].until = s.store >= 0 ? q.nsteps : last_use(k);
+    d.res = regions[(size_t)best].off;
+    if (s.store >= 0) b.s[s.store].out = d.res;
+    reg_region[dr] = best;
+    cost += (s.op == BOP_LMULT ? 24 : 2) * kncplx(kind_r[k]) / 2;
   }
-  for (int j = 0; j < q.nstreams; j++) uses_d = uses_d || q.stream[j].kind == BK_D;
-  for (int k = 0; k < q.nsteps; k++)
-    uses_d = uses_d || b.st[k].kind_r == BK_D || b.st[k].kind_a == BK_D || b.st[k].kind_b == BK_D;
-  if (off > stage_bytes) stage_bytes = off;
-  if (oo > out_slice_bytes) out_slice_bytes = oo;
+  if (fixed > fixed_bytes) fixed_bytes = fixed;
+  if (stage > stage_bytes) stage_bytes = stage;
   return true;
-}
-
-// the catalogue shape that every field's program has, or SH_GENERIC
-template <class... SS>
-static bool has_shape(const BField& b, Shape<SS...>) {
-  constexpr int ops[] = {SS::op...}, ka[] = {SS::ka...}, kb[] = {SS::kb...}, aa[] = {SS::adja...},
-                ab[] = {SS::adjb...}, sa[] = {SS::sa...}, sb[] = {SS::sb...}, eq[] = {SS::eqop...};
-  if (b.nsteps != (int)sizeof...(SS)) return false;
-  for (int k = 0; k < b.nsteps; k++) {
-    const BStep& d = b.st[k];
-    if (d.op != ops[k] || d.kind_a != ka[k] || (d.op == BOP_LMULT && d.kind_b != kb[k]) || d.adja != aa[k] ||
-        d.adjb != ab[k] || d.src_a != sa[k] || d.src_b != sb[k] || (eq[k] >= 0 && d.eqop != eq[k]))
-      return false;
-  }
-  return true;
-}
-static int shape_of(const BField& b) {
-  if (has_shape(b, ShapeConfig4{})) return SH_CONFIG4;
-  if (has_shape(b, ShapeHop{})) return SH_HOP;
-  if (has_shape(b, ShapeAxpyMaD{})) return SH_AXPY_MAD;
-  if (has_shape(b, ShapeMMaCopy{})) return SH_MMA_COPY;
-  return SH_GENERIC;
-}
-// sets each field's shape; returns the shape all fields share, SH_MULTI when
-// every field has a catalogue shape but not the same one, else SH_GENERIC
-static int common_shape(BField* h, int nfields) {
-  int common = -1;
-  bool all_known = true;
-  for (int f = 0; f < nfields; f++) {
-    h[f].shape = shape_of(h[f]);
-    all_known = all_known && h[f].shape != SH_GENERIC;
-    common = (common < 0 || common == h[f].shape) ? h[f].shape : SH_MULTI;
-  }
-  if (!all_known || common < 0) return SH_GENERIC;
-  return common;
-}
-static const void* batch_kernel_for(const BatchPlan* plan) {
-  switch (plan->shape) {
-    case SH_CONFIG4: return reinterpret_cast<const void*>(&batch_program_kernel<9, ShapeConfig4>);
-    case SH_HOP: return reinterpret_cast<const void*>(&batch_program_kernel<12, ShapeHop>);
-    case SH_AXPY_MAD: return reinterpret_cast<const void*>(&batch_program_kernel<12, ShapeAxpyMaD>);
-    case SH_MMA_COPY: return reinterpret_cast<const void*>(&batch_program_kernel<9, ShapeMMaCopy>);
-    case SH_MULTI:
-      return plan->mc == 12 ? reinterpret_cast<const void*>(&batch_program_kernel<12, MultiShape>)
-                            : reinterpret_cast<const void*>(&batch_program_kernel<9, MultiShape>);
-    default:
-      return plan->mc == 12 ? reinterpret_cast<const void*>(&batch_program_kernel<12, GenericShape>)
-                            : reinterpret_cast<const void*>(&batch_program_kernel<9, GenericShape>);
-  }
 }
 
 static BatchPlan* make_plan(const char* who, const qlagpu_F3_batch_program* fields, int nfields) {
@@ -989,69 +696,105 @@ static BatchPlan* make_plan(const char* who, const qlagpu_F3_batch_program* fiel
     set_error(QLAGPU_ERR_ARG, who, "need 1 <= nfields <= 1024 and a field table");
     return nullptr;
   }
-  int t = 128, st = 2;
-  if (!tuned_shape("F3_batch_program", &t, &st) || (t != 64 && t != 128)) {
-    t = 128;  // the kernel's launch bounds allow 64 or 128 sites per tile
-    st = 2;
-  }
+  int t = 128, st = 0;  // threads per block (the table's stages do not apply here)
+  if (!tuned_shape("F3_batch_program", &t, &st) || (t != 64 && t != 128)) t = 128;
   std::vector<BField> h((size_t)nfields);
-  unsigned stage_bytes = 0, out_slice = 0;
-  bool spills = false, uses_d = false;
+  std::vector<long long> cost((size_t)nfields);  // of a tile
+  unsigned fixed_bytes = 0, stage_bytes = 0;
   long long tiles = 0;
+  double total = 0.0;
   for (int f = 0; f < nfields; f++) {
-    if (!build_field(who, f, fields[f], t, h[(size_t)f], stage_bytes, out_slice, spills, uses_d)) return nullptr;
+    if (!build_field(who, f, fields[f], h[(size_t)f], fixed_bytes, stage_bytes, cost[(size_t)f])) return nullptr;
     h[(size_t)f].tile0 = tiles;
-    tiles += (fields[f].n + t - 1) / t;
+    const long long ft = (fields[f].n + 31) / 32;
+    tiles += ft;
+    total += (double)ft * (double)cost[(size_t)f];
   }
-  stage_bytes = (stage_bytes + 127u) & ~127u;
-  if (stage_bytes == 0) stage_bytes = 128;
-  out_slice = (out_slice + 127u) & ~127u;
-  auto smem_for = [&](int stages) {
-    return 256 + 8 * (size_t)kMaxFields + (size_t)stages * stage_bytes + (size_t)(t / 32) * out_slice +
-           (spills ? 2 * 12 * 8 * (size_t)t : 0) + 16 * (size_t)kDescWords * (t / 32 + 1);
-  };
-  size_t smem = smem_for(st);
-  while (smem > 225u * 1024u && st > 2) smem = smem_for(--st);  // shed stages before giving up
-  if (smem > 225u * 1024u) {
-    set_error(QLAGPU_ERR_ARG, who, "the programs' streams need more shared memory per tile than a block has");
-    return nullptr;
-  }
-  const int shape = common_shape(h.data(), nfields);  // also each field's own shape
   if (!device_error_word()) return nullptr;  // allocate it now, not inside a later capture
   BatchPlan* plan = new BatchPlan();
   plan->nfields = nfields;
   plan->ntiles = tiles;
-  plan->threads = t;
-  plan->stages = st;
+  plan->fixed_bytes = fixed_bytes;
   plan->stage_bytes = stage_bytes;
-  plan->out_slice_bytes = out_slice;
-  plan->spill_regs = spills ? 1 : 0;
-  plan->mc = uses_d ? 12 : 9;
-  plan->shape = shape;
-  plan->smem = smem;
-  if (cudaMalloc(&plan->dfields, sizeof(BField) * (size_t)nfields) != cudaSuccess ||
-      cudaMemcpy(plan->dfields, h.data(), sizeof(BField) * (size_t)nfields, cudaMemcpyHostToDevice) !=
-          cudaSuccess) {
+  // Two stages hide a tile's copies behind the one before it; one stage leaves
+  // room for more warps, up to the 16 that the registers allow on an SM.  Two
+  // where they still leave 16.  Measured on B200, two stages / one: 64 fields
+  // of config 4's pair 500 us (16 warps) / 576 us (16); 30 fields of a Wilson
+  // hop direction 205 (12) / 191 (16); five programs in one plan 356 (12) / 327
+  // (16).
+  const void* fn = reinterpret_cast<const void*>(&batch_program_kernel);
+  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+  int nb = 1;
+  for (plan->stages = 2;; plan->stages = 1) {
+    plan->warp_bytes =
+        (16u + 16u * (unsigned)kDescWords + fixed_bytes + (unsigned)plan->stages * stage_bytes + 127u) & ~127u;
+    plan->smem = (size_t)(t / 32) * plan->warp_bytes;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, t, plan->smem) != cudaSuccess) nb = 0;
+    cudaGetLastError();
+    if (plan->stages == 1 || nb * (t / 32) >= 16) break;
+  }
+  // very large programs: narrower blocks until one fits
+  while (nb < 1 && t > 32) {
+    t /= 2;
+    plan->smem = (size_t)(t / 32) * plan->warp_bytes;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, t, plan->smem) != cudaSuccess) nb = 0;
+    cudaGetLastError();
+  }
+  if (nb < 1) nb = 1;
+  plan->threads = t;
+  const int nw = t / 32;
+  long long grid = (long long)nb * device_sm_count();
+  if (grid * nw > tiles) grid = (tiles + nw - 1) / nw;
+  plan->grid = (int)(grid < 1 ? 1 : grid);
+  // The tiles go to the blocks in contiguous runs of equal estimated cost.
+  // Fields with one program: one run per block (its first tile pays the
+  // index and record latencies once).  Different programs: two runs each, of
+  // different parts of the list, which evens out what the cost model gets
+  // wrong.  Measured, runs per block 1 / 2 / 4: five programs in one plan 326 /
+  // 314 / 328 us, 64 fields of config 4's pair 507 / 510 / 506, 30 fields of a
+  // hop direction 189 / 197 / 202.
+  bool same = true;
+  for (int f = 1; f < nfields; f++) {
+    const BField &x = h[0], &y = h[(size_t)f];
+    same = same && x.nsteps == y.nsteps;
+    for (int k = 0; same && k < x.nsteps; k++) same = x.st[k].code == y.st[k].code;
+  }
+  const long long runs = (long long)plan->grid * (same || tiles < 16LL * plan->grid * nw ? 1 : 2);
+  plan->runs = (int)runs;
+  std::vector<long long> start((size_t)runs + 1);
+  {
+    int f = 0;
+    double before = 0.0;  // cost of the fields before f
+    for (long long w = 0; w < runs; w++) {
+      const double want = total * (double)w / (double)runs;
+      while (f + 1 < nfields) {
+        const double here = (double)((h[(size_t)f].n + 31) / 32) * (double)cost[(size_t)f];
+        if (before + here > want) break;
+        before += here;
+        f++;
+      }
+      const double c = (double)(cost[(size_t)f] > 0 ? cost[(size_t)f] : 1);
+      long long g = h[(size_t)f].tile0 + (long long)((want - before) / c);
+      if (g > tiles) g = tiles;
+      if (w > 0 && g < start[(size_t)w - 1]) g = start[(size_t)w - 1];
+      start[(size_t)w] = g;
+    }
+    start[0] = 0;
+    start[(size_t)runs] = tiles;
+  }
+  const size_t fb = sizeof(BField) * (size_t)nfields, sb = sizeof(long long) * start.size();
+  char* table = nullptr;
+  if (cudaMalloc(&table, fb + sb) != cudaSuccess ||
+      cudaMemcpy(table, h.data(), fb, cudaMemcpyHostToDevice) != cudaSuccess ||
+      cudaMemcpy(table + fb, start.data(), sb, cudaMemcpyHostToDevice) != cudaSuccess) {
     check_launch(who);
     set_error(QLAGPU_ERR_ALLOC, who, "plan table allocation failed");
-    cudaFree(plan->dfields);
+    cudaFree(table);
     delete plan;
     return nullptr;
   }
-  const void* fn = batch_kernel_for(plan);
-  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan->smem);
-  int nb = 1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, t + 32, plan->smem) != cudaSuccess || nb < 1) nb = 1;
-  cudaGetLastError();
-  long long grid = (long long)nb * device_sm_count();
-  if (grid > tiles) grid = tiles;
-  plan->grid = (int)(grid < 1 ? 1 : grid);
-  // Tile groups, measured on B200 (64 uneven fields, fraction of HBM peak by
-  // group size 1 / 4 / 8 / 16 / one contiguous run per block): config 4's
-  // shape 0.78 / 0.83 / 0.86 / 0.88 / 0.91, where each tile's work is short
-  // and a descriptor reload per tile shows; the hop shape 0.67 / 0.72 / 0.73 /
-  // 0.72 / 0.74 and a config-4 / hop mix 0.37 / 0.38 / 0.39 / 0.38 / 0.39.
-  plan->chunk = shape == SH_CONFIG4 ? (tiles + plan->grid - 1) / plan->grid : 8;
+  plan->dfields = reinterpret_cast<BField*>(table);
+  plan->dstart = reinterpret_cast<long long*>(table + fb);
   return plan;
 }
 
@@ -1104,18 +847,17 @@ extern "C" QLAB_EXPORT int qlagpu_batch_run(void* handle) {
   if (plan->ntiles == 0) return QLAGPU_OK;
   BatchParams p;
   p.fields = plan->dfields;
+  p.start = plan->dstart;
   p.nfields = plan->nfields;
-  p.ntiles = plan->ntiles;
-  p.stages = plan->stages;
+  p.fixed_bytes = plan->fixed_bytes;
   p.stage_bytes = plan->stage_bytes;
-  p.out_slice_bytes = plan->out_slice_bytes;
-  p.spill_regs = plan->spill_regs;
-  p.chunk = plan->chunk;
+  p.warp_bytes = plan->warp_bytes;
+  p.stages = plan->stages;
+  p.runs = plan->runs;
   p.err = device_error_word();
   void* args[] = {&p};
-  const void* fn = batch_kernel_for(plan);
-  if (cudaLaunchKernel(fn, dim3((unsigned)plan->grid),
-                       dim3((unsigned)plan->threads + 32u), args, plan->smem, current_stream()) != cudaSuccess) {
+  if (cudaLaunchKernel(reinterpret_cast<const void*>(&batch_program_kernel), dim3((unsigned)plan->grid),
+                       dim3((unsigned)plan->threads), args, plan->smem, current_stream()) != cudaSuccess) {
     check_launch("qlagpu_batch_run");
     return QLAGPU_ERR_LAUNCH;
   }

@@ -8,7 +8,7 @@ i = int32 index stream, r = destination read by peq/meq) it times every
 (consumer threads = sites per tile in {64,128,256}) x (pipeline stages in
 {2,3,4}) shape with CUDA events on fields larger than L2 and writes the
 fastest per key; the batched program launch (key F3_batch_program, config 4's
-64 uneven fields) over sites per tile in {64,128} x stages {2,3,4}.  libqla_b200.so reads the table at its first launch (the
+64 uneven fields) over threads per block in {64,128}.  libqla_b200.so reads the table at its first launch (the
 file beside the package, or $QLA_B200_TUNE); keys missing from it use the
 built-in heuristic.
 """
@@ -86,10 +86,10 @@ def _workloads(torch, L):
 
 class _Batch:
     """Config 4's batched launch: 64 F3 fields with extents drawn from
-    {8,12,16,20,24,32}^4, each running r = u * u2[nbr], w = r * v.  The tile
+    {8,12,16,20,24,32}^4, each running r = u * u2[nbr], w = r * v.  The block
     shape is fixed when a plan is built, so prepare() rebuilds the plan after
     each tuned shape is set."""
-    SHAPES = list(itertools.product([64, 128], [2, 3, 4]))  # the batch kernel's launch bounds allow 64 / 128
+    SHAPES = [(64, 2), (128, 2)]  # threads per block; the kernel chooses its stages from the plan
 
     def __init__(self, torch):
         import numpy as np
