@@ -454,8 +454,23 @@ __device__ __forceinline__ void coop_store(const unsigned char* slots, char* add
   }
 }
 
+// Operators whose arithmetic outweighs their bytes (specialised beside them)
+// run on this kernel too: every thread computes, and up to 255 registers each.
 template <class OP>
-__global__ void __launch_bounds__(128) site_coop_kernel(const SiteParams p) {
+struct ComputeBound {
+  static constexpr bool value = false;
+};
+// Blocks of 128 threads an SM must hold, by the 32-bit registers that one
+// site's records fill: 5 (102 registers), 3 (168) or 1 (255).  (Left to itself
+// the compiler spills the 8-colour matrix products: 211 us against 55.)
+template <class OP>
+constexpr int coop_min_blocks() {
+  constexpr int live = (OP::N0 + OP::N1 + OP::N2 + OP::NOUT) * (int)sizeof(Cx<typename OP::R>) / 4;
+  return ComputeBound<OP>::value || live > 160 ? 1 : live > 70 ? 3 : 5;
+}
+
+template <class OP>
+__global__ void __launch_bounds__(128, coop_min_blocks<OP>()) site_coop_kernel(const SiteParams p) {
   using R = typename OP::R;
   using L = CoopLayout<OP>;
   constexpr int NA = ArrN<OP::NACC>::value, C = (int)sizeof(Cx<R>);

@@ -43,39 +43,53 @@ inline LaunchShape default_shape(unsigned bytes_per_site, unsigned out_bytes) {
   return s;
 }
 
+// resident blocks per SM of a kernel at a block shape (cached)
+inline int launch_blocks_per_sm(const void* fn, int threads, size_t smem) {
+  static std::mutex mu;
+  static std::map<std::tuple<int, int, size_t, const void*>, int> cache;
+  const int dev = current_device();
+  auto key = std::make_tuple(dev, threads, smem, fn);
+  std::lock_guard<std::mutex> g(mu);
+  auto it = cache.find(key);
+  if (it != cache.end()) return it->second;
+  int nb = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, threads, smem) != cudaSuccess) nb = 1;
+  if (nb < 1) nb = 1;
+  cache[key] = nb;
+  return nb;
+}
+
+// raises a kernel's dynamic shared-memory limit to at least `smem`
+inline void launch_smem_limit(const void* fn, size_t smem) {
+  static std::mutex mu;
+  static std::map<std::pair<int, const void*>, size_t> done;
+  const int dev = current_device();
+  std::lock_guard<std::mutex> g(mu);
+  size_t& cur = done[std::make_pair(dev, fn)];
+  if (smem > cur) {
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cur = smem;
+  }
+}
+
+// Lanes that meet on one bank when each reads its own record of a flat tile
+// with 16-B accesses (8 lanes a phase, 4 banks each).
+constexpr int bank_ways(int rec_bytes) {
+  if (rec_bytes == 0 || rec_bytes % 16 != 0) return 1;  // 8-B accesses of an odd length: none
+  int u = rec_bytes / 16, w = 1;
+  while (w < 8 && u % 2 == 0) {
+    u /= 2;
+    w *= 2;
+  }
+  return w;
+}
+
 template <class OP>
 struct SiteLauncher {
   using R = typename OP::R;
   static constexpr int RB[3] = {OP::N0 * (int)sizeof(Cx<R>), OP::N1 * (int)sizeof(Cx<R>),
                                 OP::N2 * (int)sizeof(Cx<R>)};
   static constexpr int OB = OP::NOUT * (int)sizeof(Cx<R>);
-
-  static int blocks_per_sm(const void* fn, int threads, size_t smem) {
-    static std::mutex mu;
-    static std::map<std::tuple<int, int, size_t, const void*>, int> cache;
-    const int dev = current_device();
-    auto key = std::make_tuple(dev, threads, smem, fn);
-    std::lock_guard<std::mutex> g(mu);
-    auto it = cache.find(key);
-    if (it != cache.end()) return it->second;
-    int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, threads, smem) != cudaSuccess) nb = 1;
-    if (nb < 1) nb = 1;
-    cache[key] = nb;
-    return nb;
-  }
-
-  static void set_smem_attr(const void* fn, size_t smem) {
-    static std::mutex mu;
-    static std::map<std::pair<int, const void*>, size_t> done;
-    const int dev = current_device();
-    std::lock_guard<std::mutex> g(mu);
-    size_t& cur = done[std::make_pair(dev, fn)];
-    if (smem > cur) {
-      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      cur = smem;
-    }
-  }
 
   // kernel_id names the OP for the autotuner table
   static void run(SiteParams p, const char* kernel_id, void* host_result = nullptr, size_t result_bytes = 0) {
@@ -93,13 +107,23 @@ struct SiteLauncher {
     }
     p.err = device_error_word();
     // ---- path selection
-    bool direct = (p.gang != nullptr);
+    bool direct = (p.gang != nullptr);  // the warp-cooperative kernel
     for (int j = 0; j < OP::NIN; j++) {
       const Opnd& o = p.in[j];
       const void* q = o.mode == OM_PTR ? (const void*)o.ptrs : (o.mode == OM_IDX ? (const void*)o.idx : o.base);
       if (!aligned16(q)) direct = true;
     }
     if (OP::NOUT > 0 && !aligned16(p.out)) direct = true;
+    // Records of a multiple of 128 B (4 and 8 colours' matrices and Dirac
+    // fermions) lie flat in a bulk-copied tile with all eight lanes of a phase
+    // on the same banks; the warp-cooperative kernel pads its slots.  Measured
+    // (tile / padded slots, us): QLA_FN_M_veq_M_times_Ma nc = 4 on 320,000 sites
+    // 41 / 24, nc = 8 on 41,472 sites 253 / 48; QLA_DFN_c_veq_D_dot_D nc = 4 32 /
+    // 23.  Up to four ways (D3 Dirac fermions) the copies still bound the tile.
+    if (bank_ways(OB) == 8) direct = true;
+    for (int j = 0; j < OP::NIN; j++)
+      if (p.in[j].mode == OM_CONTIG && bank_ways(RB[j]) == 8) direct = true;
+    if (ComputeBound<OP>::value) direct = true;
 
     // ---- reduction scratch / result destination
     ReduceScratch* rs = nullptr;
@@ -120,9 +144,9 @@ struct SiteLauncher {
       while (nw > 1 && nw * wb > 48u * 1024u) nw /= 2;
       const size_t smem = (size_t)nw * wb;
       const void* fn = reinterpret_cast<const void*>(&site_coop_kernel<OP>);
-      set_smem_attr(fn, smem);
+      launch_smem_limit(fn, smem);
       long long grid = (p.n + 32 * nw - 1) / (32 * nw);
-      const long long cap = (long long)blocks_per_sm(fn, 32 * nw, smem) * sms;
+      const long long cap = (long long)launch_blocks_per_sm(fn, 32 * nw, smem) * sms;
       if (grid > cap) grid = cap;
       if (reduce && grid > rs->max_blocks) grid = rs->max_blocks;
       void* args[] = {&p};
@@ -182,8 +206,8 @@ struct SiteLauncher {
       p.stages = sh.stages;
       const size_t smem = tma_smem_bytes(T, p.stages, p.stage_bytes, OB);
       const void* fn = reinterpret_cast<const void*>(&site_tma_kernel<OP>);
-      set_smem_attr(fn, smem);
-      const int nb = blocks_per_sm(fn, T + 32, smem);
+      launch_smem_limit(fn, smem);
+      const int nb = launch_blocks_per_sm(fn, T + 32, smem);
       long long grid = (long long)nb * sms;
       if (grid > p.ntiles) grid = p.ntiles;
       if (grid < 1) grid = 1;

@@ -72,7 +72,7 @@ static unsigned char* scratch_on_current_device() {
       cudaGetLastError();
       return nullptr;
     }
-    SiteLauncher<Op>::set_smem_attr(reinterpret_cast<const void*>(&site_tma_kernel<Op>), tile_smem_bytes());
+    launch_smem_limit(reinterpret_cast<const void*>(&site_tma_kernel<Op>), tile_smem_bytes());
     if (cudaGetLastError() != cudaSuccess) return nullptr;
     addr[dev] = static_cast<unsigned char*>(p);
   }
