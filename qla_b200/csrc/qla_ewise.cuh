@@ -330,7 +330,26 @@ inline void api_ew(const char* kid, void* r, const void* scal, Opnd s, Opnd b, O
 }
 
 // ---------------------------------------------------------------------------
-// outer product M (eqop) a b^+ of two ColorVectors (one thread per element)
+// outer product M (eqop) a b^+ of two ColorVectors: on the site engine where the
+// operands are contiguous and 16-B aligned (every record is moved once, by bulk
+// copies; one thread per element, whose factors come from two other records,
+// took 20.9 us for M_veq_V_times_Va on 24^3 x 48, so 13.0), else one thread
+// per element
+template <typename R_>
+struct OuterOp {
+  using R = R_;
+  static constexpr int NIN = 2, N0 = 3, N1 = 3, N2 = 0, NOUT = 9, NACC = 0;
+  __device__ __forceinline__ static void apply(const SiteParams& p, const Cx<R> (&a)[3], const Cx<R> (&b)[3],
+                                               const Cx<R> (&)[1], Cx<R> (&y)[9]) {
+    // c_(eqop)_c_times_ca(r, a, b): the scalar slot carries a
+#pragma unroll
+    for (int e = 0; e < 9; e++) y[e] = ew_apply<R, EW_CTA>(p.eqop, y[e], a[e / 3], b[e % 3], Cx<R>{R(0), R(0)});
+  }
+  __device__ static void accum(const SiteParams&, const Cx<R> (&)[3], const Cx<R> (&)[3], const Cx<R> (&)[1],
+                               double*) {}
+  __device__ static void finish(const SiteParams&, const double*) {}
+};
+
 template <typename R>
 __global__ void __launch_bounds__(256) outer_kernel(const EwParams p) {
   const long long total = p.n * 9;
@@ -344,7 +363,6 @@ __global__ void __launch_bounds__(256) outer_kernel(const EwParams p) {
     const Cx<R> b = rec_ptr<R>(p.c, k, 3)[e % 3];
     Cx<R>* out = static_cast<Cx<R>*>(p.out) + k * 9 + e;
     const Cx<R> x = load ? *out : Cx<R>{R(0), R(0)};
-    // c_(eqop)_c_times_ca(r, a, b): the scalar slot carries a
     *out = ew_apply<R, EW_CTA>(p.eqop, x, a, b, Cx<R>{R(0), R(0)});
   }
 }
@@ -354,6 +372,11 @@ inline void api_outer(const char* kid, void* r, Opnd a, Opnd b, const int* gang,
   if (n <= 0) return;
   if (!r || !opnd_ok(a) || !opnd_ok(b)) {
     set_error(QLAGPU_ERR_NULLPTR, kid, "NULL argument");
+    return;
+  }
+  if (gang == nullptr && a.mode == OM_CONTIG && b.mode == OM_CONTIG && aligned16(r) && aligned16(a.base) &&
+      aligned16(b.base)) {
+    api_map<OuterOp<R>>(kid, r, a, b, gang, n, eqop);
     return;
   }
   EwParams p;
@@ -380,28 +403,37 @@ enum LdKind : int { LD_DOT = 0, LD_DOT_AA = 1, LD_ADOT = 2, LD_REDOT = 3, LD_NOR
 // LD_REDOT  x += Re(conj(a_e) b_e)             (re_X_dot_X)
 // LD_NORM2  x += |a_e|^2                       (norm2_X)
 
-// The accumulation of one site shared by the two kernels below: x over the
-// elements e in order, from the records a and b (any memory space)
-template <typename R, int NE, int KIND, int PERM>
-__device__ __forceinline__ void ldot_site(const Cx<R>* a, const Cx<R>* b, double& xr, double& xi) {
+// one term of the accumulation
+template <typename R, int KIND>
+__device__ __forceinline__ void ldot_term(Cx<R> ua, Cx<R> vb, double& xr, double& xi) {
+  const double ur = ua.re, ui = ua.im, vr = vb.re, vi = vb.im;
+  if constexpr (KIND == LD_DOT || KIND == LD_REDOT || KIND == LD_NORM2) {
+    xr = __dadd_rn(xr, __dadd_rn(__dmul_rn(ur, vr), __dmul_rn(ui, vi)));
+    if constexpr (KIND == LD_DOT) xi = __dadd_rn(xi, __dsub_rn(__dmul_rn(ur, vi), __dmul_rn(ui, vr)));
+  } else if constexpr (KIND == LD_DOT_AA) {
+    xr = __dadd_rn(xr, __dsub_rn(__dmul_rn(ur, vr), __dmul_rn(ui, vi)));
+    xi = __dadd_rn(xi, __dsub_rn(__dmul_rn(-ur, vi), __dmul_rn(ui, vr)));
+  } else {
+    xr = __dadd_rn(xr, __dsub_rn(__dmul_rn(ur, vr), __dmul_rn(ui, vi)));
+    xi = __dadd_rn(xi, __dadd_rn(__dmul_rn(ur, vi), __dmul_rn(ui, vr)));
+  }
+}
+// the accumulation of one site: x over the elements e in order, from the
+// records a and b (any memory space); blk: row length of the permuted source
+template <typename R, int KIND>
+__device__ __forceinline__ void ldot_site(const Cx<R>* a, const Cx<R>* b, int ne, int blk, double& xr, double& xi) {
   xr = 0.0;
   xi = 0.0;
+  if constexpr (KIND == LD_ADOT || KIND == LD_DOT_AA) {
+    for (int x = 0; x < blk; x++)
+#pragma unroll 3
+      for (int y = 0; y < blk; y++) {
+        const int e = x * blk + y, pe = y * blk + x;
+        ldot_term<R, KIND>(a[KIND == LD_ADOT ? pe : e], b[KIND == LD_DOT_AA ? pe : e], xr, xi);
+      }
+  } else {
 #pragma unroll 4
-  for (int e = 0; e < NE; e++) {
-    Cx<R> ua = a[e], vb = b[e];
-    if constexpr (KIND == LD_ADOT) ua = a[perm_elem<PERM, NE>(e)];
-    if constexpr (KIND == LD_DOT_AA) vb = b[perm_elem<PERM, NE>(e)];
-    const double ur = ua.re, ui = ua.im, vr = vb.re, vi = vb.im;
-    if constexpr (KIND == LD_DOT || KIND == LD_REDOT || KIND == LD_NORM2) {
-      xr = __dadd_rn(xr, __dadd_rn(__dmul_rn(ur, vr), __dmul_rn(ui, vi)));
-      if constexpr (KIND == LD_DOT) xi = __dadd_rn(xi, __dsub_rn(__dmul_rn(ur, vi), __dmul_rn(ui, vr)));
-    } else if constexpr (KIND == LD_DOT_AA) {
-      xr = __dadd_rn(xr, __dsub_rn(__dmul_rn(ur, vr), __dmul_rn(ui, vi)));
-      xi = __dadd_rn(xi, __dsub_rn(__dmul_rn(-ur, vi), __dmul_rn(ui, vr)));
-    } else {
-      xr = __dadd_rn(xr, __dsub_rn(__dmul_rn(ur, vr), __dmul_rn(ui, vi)));
-      xi = __dadd_rn(xi, __dadd_rn(__dmul_rn(ur, vi), __dmul_rn(ui, vr)));
-    }
+    for (int e = 0; e < ne; e++) ldot_term<R, KIND>(a[e], b[e], xr, xi);
   }
 }
 
@@ -427,72 +459,163 @@ __device__ __forceinline__ void ldot_store(void* out, long long k, int eqop, dou
   }
 }
 
-// Staged form for contiguous operands without a gang index: a block copies
-// the records of S consecutive sites with coalesced loads (LD_U in flight
-// per thread) into shared memory (rows padded by one complex number against
-// bank conflicts), then each of the first S threads accumulates its site
-// from there.  (Per-thread cp.async copies in two stages measured slower
-// than this on B200: 0.75 against 0.88 of HBM for the D3 D dot product.)
 // one thread per site, records read where they are (gang or pointer forms)
-template <typename R, int NE, int KIND, int PERM>
-__global__ void __launch_bounds__(256) ldot_kernel(const EwParams p) {
+template <typename R, int KIND>
+__global__ void __launch_bounds__(256) ldot_kernel(const EwParams p, int ne, int blk) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < p.n;
        i += (long long)gridDim.x * blockDim.x) {
     const long long k = p.gang ? (long long)p.gang[i] : i;
-    const Cx<R>* a = rec_ptr<R>(p.b, k, NE);
-    const Cx<R>* b = (KIND == LD_NORM2) ? a : rec_ptr<R>(p.c, k, NE);
+    const Cx<R>* a = rec_ptr<R>(p.b, k, ne);
+    const Cx<R>* b = (KIND == LD_NORM2) ? a : rec_ptr<R>(p.c, k, ne);
     double xr, xi;
-    ldot_site<R, NE, KIND, PERM>(a, b, xr, xi);
+    ldot_site<R, KIND>(a, b, ne, blk, xr, xi);
     ldot_store<R, KIND>(p.out, k, p.eqop, xr, xi);
   }
 }
 
-template <typename R, int NE, int KIND, int PERM, int S>
-__global__ void __launch_bounds__(128) ldot_smem_kernel(const EwParams p) {
-  extern __shared__ __align__(16) unsigned char ldsm[];
-  constexpr int ST = NE + 1;  // padded row stride (complex numbers)
-  Cx<R>* sa = reinterpret_cast<Cx<R>*>(ldsm);
-  Cx<R>* sb = sa + S * ST;
-  const Cx<R>* A = static_cast<const Cx<R>*>(p.b.base);
-  const Cx<R>* B = static_cast<const Cx<R>*>(KIND == LD_NORM2 ? p.b.base : p.c.base);
-  const long long ntile = (p.n + S - 1) / S;
-  for (long long tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
-    const long long s0 = tile * S;
-    const int ns = (int)((p.n - s0) < S ? (p.n - s0) : S);
-    const long long base = s0 * NE;
-    const int nf = ns * NE;
-    // LD_U loads per thread issued before their shared-memory stores, so
-    // that many are in flight (a load-store loop would wait for each)
-    constexpr int LD_U = 12;
-    for (int f0 = threadIdx.x; f0 < nf; f0 += LD_U * blockDim.x) {
-      Cx<R> va[LD_U], vb[LD_U];
-#pragma unroll
-      for (int u = 0; u < LD_U; u++) {
-        const int f = f0 + u * blockDim.x;
-        if (f < nf) {
-          va[u] = A[base + f];
-          if constexpr (KIND != LD_NORM2) vb[u] = B[base + f];
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < LD_U; u++) {
-        const int f = f0 + u * blockDim.x;
-        if (f < nf) {
-          const int row = f / NE, col = f - row * NE;
-          sa[row * ST + col] = va[u];
-          if constexpr (KIND != LD_NORM2) sb[row * ST + col] = vb[u];
-        }
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x < ns) {
-      double xr, xi;
-      const Cx<R>* ra = sa + threadIdx.x * ST;
-      ldot_site<R, NE, KIND, PERM>(ra, KIND == LD_NORM2 ? ra : sb + threadIdx.x * ST, xr, xi);
-      ldot_store<R, KIND>(p.out, s0 + threadIdx.x, p.eqop, xr, xi);
-    }
-    __syncthreads();
+// Contiguous operands without a gang index: a warp takes 32 sites.
+// Their records come into the warp's shared-memory slots with bulk copies
+// (8-B cp.async where a base is not 16-B aligned or a tile is partial), each
+// lane then sums its site in the reference's order from there, and the 32
+// results leave as one coalesced store.  The per-site FP64 chain is short
+// beside the copies of the SM's other warps, so the kernel runs at the rate of
+// the copies; a block-wide tile with a barrier between copying and summing
+// left three of four warps idle while it summed P records.  Where all eight
+// lanes of a phase would meet on one bank (records of a multiple of 128 B) the
+// slots are padded by 16 B: long records (P) then come one bulk copy per lane,
+// short ones in 16-B pieces, consecutive lanes taking consecutive pieces.  The
+// record length is an argument: the fixed and the N-colour libraries share the
+// kernel.  Measured (before / after, us): QLA_F3_C_veq_D_dot_D on 24^3 x 48
+// 29.1 / 22.1, R_veq_norm2_P on an eighth of it 30.7 / 24.5;
+// QLA_FN_C_veq_D_dot_D at nc = 4 on 20^3 x 40 82 / 17.1.
+__host__ __device__ inline unsigned ldot_slot(unsigned rb) { return (rb % 128u == 0u) ? rb + 16u : rb; }
+template <typename R, int KIND>
+__global__ void __launch_bounds__(128) ldot_tile_kernel(const EwParams p, int ne, int blk, int bulk, unsigned* err) {
+  extern __shared__ __align__(128) unsigned char ldsm[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  constexpr int NOP = KIND == LD_NORM2 ? 1 : 2;
+  const unsigned rb = (unsigned)ne * (unsigned)sizeof(Cx<R>), sb = ldot_slot(rb);
+  unsigned char* mine = ldsm + (size_t)warp * (128u + NOP * 32u * sb);
+  uint64_t* bar = reinterpret_cast<uint64_t*>(mine);
+  unsigned char* slot[2] = {mine + 128, mine + 128 + (NOP - 1) * 32u * sb};
+  const char* base[2] = {static_cast<const char*>(p.b.base), static_cast<const char*>(p.c.base)};
+  if (lane == 0) {
+    mbar_init(bar, 1);
+    mbar_init_fence();
   }
+  __syncwarp();
+  // short padded records: 32 / per records at a time, a 16-B piece per lane
+  const unsigned per = rb / 16u;
+  const bool pieces = sb != rb && per <= 32u;
+  const unsigned r0 = pieces ? lane / per : 0u, pc = pieces ? lane % per : 0u, rstep = pieces ? 32u / per : 1u;
+  const unsigned rend = r0 < rstep ? 32u : 0u;
+  const long long i0 = ((long long)blockIdx.x * nw + warp) * 32;
+  if (i0 >= p.n) return;
+  const int nv = p.n - i0 < 32 ? (int)(p.n - i0) : 32;
+  if (bulk && nv == 32) {
+    if (pieces) {
+#pragma unroll
+      for (int j = 0; j < NOP; j++) {
+        const char* src = base[j] + i0 * rb + pc * 16u;
+        for (unsigned r = r0; r < rend; r += rstep) cp_async_16(slot[j] + r * sb + pc * 16u, src + r * rb);
+      }
+      cp_async_wait_all();
+      __syncwarp();
+    } else {
+      if (lane == 0) mbar_arrive_expect_tx(bar, NOP * 32u * rb);
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < NOP; j++) {
+        const char* src = base[j] + i0 * rb;
+        if (sb != rb)
+          bulk_g2s(slot[j] + lane * sb, src + lane * rb, rb, bar, policy_evict_first());
+        else if (lane == 0)
+          bulk_g2s(slot[j], src, 32u * rb, bar, policy_evict_first());
+      }
+      const bool ok = mbar_wait_bounded(bar, 0u, err);
+      if (!__all_sync(0xffffffffu, ok)) {
+        mbar_wait_bounded(bar, 0u, err, 200000000ull);  // drain before the slots are released
+        return;
+      }
+    }
+  } else {
+    // a partial tile, or a base off a 16-B boundary: 8-B copies, or 4-B ones
+    // (a QLA_F_Complex array need not start on an 8-B boundary)
+    const bool by8 = ((reinterpret_cast<uintptr_t>(base[0]) | reinterpret_cast<uintptr_t>(base[NOP - 1])) & 7u) == 0;
+    const unsigned w = by8 ? 8u : 4u, pw = rb / w, total = (unsigned)nv * pw;
+#pragma unroll
+    for (int j = 0; j < NOP; j++)
+      for (unsigned q = lane; q < total; q += 32u) {
+        unsigned char* dst = slot[j] + (q / pw) * sb + (q % pw) * w;
+        const char* src = base[j] + i0 * rb + q * w;
+        if (by8)
+          cp_async_8(dst, src);
+        else
+          cp_async_4(dst, src);
+      }
+    cp_async_wait_all();
+    __syncwarp();
+  }
+  if (lane < nv) {
+    double xr, xi;
+    const Cx<R>* a = reinterpret_cast<const Cx<R>*>(slot[0] + lane * sb);
+    const Cx<R>* b = reinterpret_cast<const Cx<R>*>(slot[NOP - 1] + lane * sb);
+    if constexpr (KIND == LD_ADOT || KIND == LD_DOT_AA) {
+      ldot_site<R, KIND>(a, b, ne, blk, xr, xi);
+    } else if (rb % 16u == 0u) {  // the same terms in the same order, 16 B per load
+      xr = 0.0;
+      xi = 0.0;
+      constexpr int CPV = 16 / (int)sizeof(Cx<R>);
+#pragma unroll 3
+      for (int v = 0; v < ne / CPV; v++) {
+        Cx<R> ua[CPV], vb[CPV];
+        load_rec<R, CPV>(ua, a + v * CPV);
+        if constexpr (KIND != LD_NORM2) load_rec<R, CPV>(vb, b + v * CPV);
+#pragma unroll
+        for (int h = 0; h < CPV; h++) ldot_term<R, KIND>(ua[h], KIND == LD_NORM2 ? ua[h] : vb[h], xr, xi);
+      }
+    } else {
+      ldot_site<R, KIND>(a, b, ne, blk, xr, xi);
+    }
+    ldot_store<R, KIND>(p.out, i0 + lane, p.eqop, xr, xi);
+  }
+}
+
+// ne complex numbers per record, blk: row length of a permuted source
+template <typename R, int KIND>
+inline void run_ldot(const char* kid, int ne, int blk, void* r, Opnd a, Opnd b, const int* gang, int n, int eqop) {
+  EwParams p;
+  std::memset(&p, 0, sizeof(p));
+  p.out = r;
+  p.b = a;
+  p.c = b;
+  p.gang = gang;
+  p.n = n;
+  p.eqop = eqop;
+  constexpr int NOP = KIND == LD_NORM2 ? 1 : 2;
+  const unsigned rb = (unsigned)ne * (unsigned)sizeof(Cx<R>);
+  const size_t warp_bytes = 128u + NOP * 32u * (size_t)ldot_slot(rb);
+  const int sms = device_sm_count();
+  // (records too long for one warp's slots -- P of many colours -- go direct)
+  if (gang == nullptr && a.mode == OM_CONTIG && (KIND == LD_NORM2 || b.mode == OM_CONTIG) &&
+      warp_bytes <= 200u * 1024u) {
+    int nw = 4;
+    while (nw > 1 && nw * warp_bytes > 56u * 1024u) nw /= 2;
+    const size_t smem = (size_t)nw * warp_bytes;
+    const void* fn = reinterpret_cast<const void*>(&ldot_tile_kernel<R, KIND>);
+    launch_smem_limit(fn, 227 * 1024);
+    // one tile per warp: the copies of the blocks that follow fill the SM while
+    // the present ones sum (persistent warps of two or three tiles each ended
+    // unevenly: norm2_D 20 us, 13 so)
+    const long long grid = ((long long)n + 32 * nw - 1) / (32 * nw);
+    const int bulk = aligned16(a.base) && (KIND == LD_NORM2 || aligned16(b.base)) ? 1 : 0;
+    ldot_tile_kernel<R, KIND><<<(unsigned)grid, 32 * nw, smem, current_stream()>>>(p, ne, blk, bulk, device_error_word());
+  } else {
+    long long grid = ((long long)n + 255) / 256;
+    if (grid > (long long)sms * 16) grid = (long long)sms * 16;
+    ldot_kernel<R, KIND><<<(unsigned)(grid < 1 ? 1 : grid), 256, 0, current_stream()>>>(p, ne, blk);
+  }
+  check_launch(kid);
 }
 
 template <typename R, int NE, int KIND, int PERM>
@@ -502,34 +625,7 @@ inline void api_ldot(const char* kid, void* r, Opnd a, Opnd b, const int* gang, 
     set_error(QLAGPU_ERR_NULLPTR, kid, "NULL argument");
     return;
   }
-  EwParams p;
-  std::memset(&p, 0, sizeof(p));
-  p.out = r;
-  p.b = a;
-  p.c = b;
-  p.gang = gang;
-  p.n = n;
-  p.eqop = eqop;
-  const long long cap = (long long)device_sm_count() * 16;
-  if (gang == nullptr && a.mode == OM_CONTIG && (KIND == LD_NORM2 || b.mode == OM_CONTIG)) {
-    constexpr int S = NE > 32 ? 32 : 128;
-    const size_t smem = (size_t)(KIND == LD_NORM2 ? 1 : 2) * S * (NE + 1) * sizeof(Cx<R>);
-    const void* fn = reinterpret_cast<const void*>(&ldot_smem_kernel<R, NE, KIND, PERM, S>);
-    static bool attr_set[64] = {false};
-    const int dev = current_device();
-    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      attr_set[dev] = true;
-    }
-    long long grid = ((long long)n + S - 1) / S;
-    if (grid > cap) grid = cap;
-    ldot_smem_kernel<R, NE, KIND, PERM, S><<<(unsigned)(grid < 1 ? 1 : grid), 128, smem, current_stream()>>>(p);
-  } else {
-    long long grid = ((long long)n + 255) / 256;
-    if (grid > cap) grid = cap;
-    ldot_kernel<R, NE, KIND, PERM><<<(unsigned)(grid < 1 ? 1 : grid), 256, 0, current_stream()>>>(p);
-  }
-  check_launch(kid);
+  run_ldot<R, KIND>(kid, NE, PERM == PERM_P ? 12 : PERM == PERM_M ? 3 : 1, r, a, b, gang, n, eqop);
 }
 
 }  // namespace qlab

@@ -208,50 +208,7 @@ inline void api_outer_n(const char* kid, int nc, void* r, Opnd a, Opnd b, const 
 }
 
 // ---------------------------------------------------------------------------
-// site-local dot products and norms: ldot_site's accumulation with run-time
-// record length; the permuted forms walk the transposed source row by row
-template <typename R, int KIND>
-__device__ __forceinline__ void ldot_site_n(const Cx<R>* a, const Cx<R>* b, const NcDims& d, double& xr,
-                                            double& xi) {
-  xr = 0.0;
-  xi = 0.0;
-  const bool perm = (KIND == LD_ADOT || KIND == LD_DOT_AA);
-  const int B = perm ? d.blk : 1;
-  const int rows = perm ? d.blk : 1, cols = perm ? d.blk : d.ne;
-  for (int x = 0; x < rows; x++)
-    for (int y = 0; y < cols; y++) {
-      const int e = x * cols + y;
-      const int pe = perm ? y * B + x : e;
-      Cx<R> ua = a[e], vb = b[e];
-      if constexpr (KIND == LD_ADOT) ua = a[pe];
-      if constexpr (KIND == LD_DOT_AA) vb = b[pe];
-      const double ur = ua.re, ui = ua.im, vr = vb.re, vi = vb.im;
-      if constexpr (KIND == LD_DOT || KIND == LD_REDOT || KIND == LD_NORM2) {
-        xr = __dadd_rn(xr, __dadd_rn(__dmul_rn(ur, vr), __dmul_rn(ui, vi)));
-        if constexpr (KIND == LD_DOT) xi = __dadd_rn(xi, __dsub_rn(__dmul_rn(ur, vi), __dmul_rn(ui, vr)));
-      } else if constexpr (KIND == LD_DOT_AA) {
-        xr = __dadd_rn(xr, __dsub_rn(__dmul_rn(ur, vr), __dmul_rn(ui, vi)));
-        xi = __dadd_rn(xi, __dsub_rn(__dmul_rn(-ur, vi), __dmul_rn(ui, vr)));
-      } else {
-        xr = __dadd_rn(xr, __dsub_rn(__dmul_rn(ur, vr), __dmul_rn(ui, vi)));
-        xi = __dadd_rn(xi, __dadd_rn(__dmul_rn(ur, vi), __dmul_rn(ui, vr)));
-      }
-    }
-}
-
-template <typename R, int KIND>
-__global__ void __launch_bounds__(256) ldotn_kernel(const EwParams p, const NcDims d) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < p.n;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long k = p.gang ? (long long)p.gang[i] : i;
-    const Cx<R>* a = rec_ptr<R>(p.b, k, d.ne);
-    const Cx<R>* b = (KIND == LD_NORM2) ? a : rec_ptr<R>(p.c, k, d.ne);
-    double xr, xi;
-    ldot_site_n<R, KIND>(a, b, d, xr, xi);
-    ldot_store<R, KIND>(p.out, k, p.eqop, xr, xi);
-  }
-}
-
+// site-local dot products and norms (run_ldot takes any record length)
 template <typename R, int KIND>
 inline void api_ldot_n(const char* kid, int nc, int ne, int perm, void* r, Opnd a, Opnd b, const int* gang, int n,
                        int eqop) {
@@ -260,16 +217,7 @@ inline void api_ldot_n(const char* kid, int nc, int ne, int perm, void* r, Opnd 
     set_error(QLAGPU_ERR_NULLPTR, kid, "NULL argument");
     return;
   }
-  EwParams p;
-  std::memset(&p, 0, sizeof(p));
-  p.out = r;
-  p.b = a;
-  p.c = b;
-  p.gang = gang;
-  p.n = n;
-  p.eqop = eqop;
-  ldotn_kernel<R, KIND><<<nc_grid(n), 256, 0, current_stream()>>>(p, nc_dims(nc, ne, perm));
-  check_launch(kid);
+  run_ldot<R, KIND>(kid, ne, nc_dims(nc, ne, perm).blk, r, a, b, gang, n, eqop);
 }
 
 // ---------------------------------------------------------------------------
@@ -597,7 +545,7 @@ __global__ void __launch_bounds__(256) gdotn_kernel(const EwParams p, const Site
     const Cx<R>* a = rec_ptr<R>(p.b, k, d.ne);
     const Cx<R>* b = (KIND == LD_NORM2) ? a : rec_ptr<R>(p.c, k, d.ne);
     double xr, xi;
-    ldot_site_n<R, KIND>(a, b, d, xr, xi);
+    ldot_site<R, KIND>(a, b, d.ne, d.blk, xr, xi);
     dd_add(acc[0], xr);
     if constexpr (FIN::NACC > 1) dd_add(acc[1], xi);
   }

@@ -576,7 +576,7 @@ __global__ void __launch_bounds__(128) gdot_kernel(const EwParams p, const SiteP
     const Cx<R>* a = rec_ptr<R>(p.b, k, NE);
     const Cx<R>* b = (KIND == LD_NORM2) ? a : rec_ptr<R>(p.c, k, NE);
     double xr, xi;
-    ldot_site<R, NE, KIND, PERM>(a, b, xr, xi);
+    ldot_site<R, KIND>(a, b, NE, PERM == PERM_P ? 12 : PERM == PERM_M ? 3 : 1, xr, xi);
     dd_add(acc[0], xr);
     if constexpr (FIN::NACC > 1) dd_add(acc[1], xi);
   }

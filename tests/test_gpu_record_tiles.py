@@ -1,0 +1,116 @@
+"""Kernels that take 32 sites of a contiguous field per warp -- the site-local
+products, the random fills -- and the padded-slot products of 4 and 8 colours,
+at the edges of their tiles and for fields that start off a 16-B boundary,
+against the oracle."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import qla_testlib as T
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [1, 31, 32, 33, 127, 129, 1000]
+LOCAL = ["C_veq_V_dot_V", "C_vpeq_D_dot_D", "R_veq_norm2_P", "R_vmeq_re_M_dot_M", "C_veq_M_dot_Ma", "C_veqm_Pa_dot_P",
+         "R_veq_norm2_H", "C_veq_Ma_dot_M", "M_vpeq_V_times_Va"]
+
+
+def _shifted(cuda, arr, off):
+    """Device copy of arr that starts `off` bytes past a 16-B boundary: (address, tensor)."""
+    raw = np.ascontiguousarray(arr).view(np.uint8).reshape(-1)
+    t = cuda.zeros(raw.size + 32, dtype=cuda.uint8, device="cuda")
+    t[off:off + raw.size] = cuda.from_numpy(raw.copy()).cuda()
+    return t.data_ptr() + off, t
+
+
+def _back(t, off, like):
+    raw = t[off:off + like.nbytes].cpu().numpy()
+    return raw.view(like.dtype).reshape(like.shape)
+
+
+def _call(qla, cuda, name, lead, e, ins, n, off):
+    args, keep, r = list(lead), [], None
+    for t, p in zip(e["ctypes"], e["params"]):
+        if p == "n":
+            args.append(n)
+            continue
+        a, dev = _shifted(cuda, ins[p][2], off)
+        keep.append(dev)
+        args.append(ctypes.c_void_p(a))
+        if p == "r":
+            r = dev
+    getattr(qla.lib(), name)(*args)
+    qla.check(name)
+    return _back(r, off, ins["r"][2])
+
+
+@pytest.mark.parametrize("pc,nc", [("F3", 3), ("D3", 3), ("FN", 2), ("FN", 4), ("DN", 2), ("DN", 4)])
+def test_site_local_products(qla, cuda, pc, nc):
+    byname = {e["name"]: e for e in qla.manifest()}
+    rng = np.random.default_rng(31 + nc)
+    dt = np.float32 if pc[0] == "F" else np.float64
+    for n in SIZES:
+        for short in LOCAL:
+            name = f"QLA_{pc}_{short}"
+            e = byname[name if nc == 3 else T.fixed_colour_twin(name)]
+            ins, idx, gang = T.ewise_inputs(e, rng, dt, n, n, nc=nc)
+            want = T.ewise_oracle(e, ins, idx, gang, n, nc=nc)
+            for off in (0, 8, 4) if dt == np.float32 else (0, 8):  # bytes past a 16-B boundary
+                got = _call(qla, cuda, name, [] if nc == 3 else [nc], e, ins, n, off)
+                assert T.bits_equal(got, want), (name, n, off)
+
+
+@pytest.mark.parametrize("pc,dest", [("F3", "V"), ("F3", "D"), ("F3", "P"), ("D3", "V"), ("D3", "M"), ("F", "R"),
+                                     ("F", "C"), ("D", "R")])
+@pytest.mark.parametrize("op", ["gaussian", "random"])
+def test_random_fills(qla, cuda, pc, dest, op):
+    if op == "random" and dest != "R":
+        pytest.skip("uniform fills exist for real fields only")
+    byname = {e["name"]: e for e in qla.manifest()}
+    name = f"QLA_{pc}_{dest}_veq_{op}_S"
+    e = byname[name]
+    rng = np.random.default_rng(77)
+    for n in SIZES:
+        ins, idx, gang, ints, want_r, want_s = T.random_case(e, rng, n, n)
+        for off_r, off_s in ((0, 0), (8, 4), (0, 12)):
+            ra, rt = _shifted(cuda, ins["r"][2], off_r)
+            sa, st = _shifted(cuda, ins["a"][2], off_s)
+            getattr(qla.lib(), name)(ctypes.c_void_p(ra), ctypes.c_void_p(sa), n)
+            qla.check(name)
+            assert T.bits_equal(_back(st, off_s, want_s), want_s), (name, n, off_s)
+            got = np.asarray(_back(rt, off_r, want_r), np.float32).ravel()
+            w = np.asarray(want_r, np.float32).ravel()
+            if op == "random":
+                assert T.bits_equal(got, w), (name, n)
+            else:  # the stated bound: one float ulp
+                assert np.all(np.abs(got.astype(np.float64) - w) <= np.spacing(np.abs(w))), (name, n)
+
+
+@pytest.mark.parametrize("pc", ["FN", "DN"])
+@pytest.mark.parametrize("nc", [2, 4, 8])
+def test_padded_slot_products(qla, cuda, pc, nc):
+    rng = np.random.default_rng(nc)
+    dt = np.float32 if pc == "FN" else np.float64
+    L = qla.lib()
+    for n in (1, 31, 33, 129, 515):
+        a = T.gaussian_field(rng, n, nc * nc, dt)
+        b, v = T.gaussian_field(rng, n, nc * nc, dt), T.gaussian_field(rng, n + 3, nc, dt)
+        d, d2 = T.gaussian_field(rng, n, 4 * nc, dt), T.gaussian_field(rng, n, 4 * nc, dt)
+        idx = rng.integers(0, n + 3, n).astype(np.int32)
+        ad, bd, vd, xd = T.to_dev(a), T.to_dev(b), T.to_dev(v), T.to_dev(idx)
+        rm, rv = T.to_dev(np.zeros_like(a)), T.to_dev(np.zeros((n, 2 * nc), dt))
+        getattr(L, f"QLA_{pc}_M_veq_M_times_Ma")(nc, T.ptr_dev(rm), T.ptr_dev(ad), T.ptr_dev(bd), n)
+        getattr(L, f"QLA_{pc}_V_eq_M_times_xV")(nc, T.ptr_dev(rv), T.ptr_dev(ad), T.ptr_dev(vd), T.ptr_dev(xd), n)
+        wm, wv = np.zeros_like(a), np.zeros((n, 2 * nc), dt)
+        T.ora_lmult(wm, a, b, n, nc, "eq", adjb=1, nc=nc)
+        T.ora_lmult(wv, a, v, n, 1, "eq", idx_b=idx, nc=nc)
+        assert T.bits_equal(T.to_host(rm), wm) and T.bits_equal(T.to_host(rv), wv), (nc, n)
+        res = cuda.zeros(2, dtype=cuda.float64, device="cuda")
+        dd, d2d = T.to_dev(d), T.to_dev(d2)
+        getattr(L, "QLA_DFN_c_veq_D_dot_D" if pc == "FN" else "QLA_DN_c_veq_D_dot_D")(
+            nc, T.ptr_dev(res), T.ptr_dev(dd), T.ptr_dev(d2d), n)
+        z, z2 = (x.astype(np.float64).ravel().view(np.complex128) for x in (d, d2))
+        got = complex(*res.cpu().tolist())
+        assert abs(got - np.vdot(z, z2)) <= 1e-12 * np.abs(z).sum() * np.abs(z2).max(), (nc, n)
+    qla.check("padded slots")
