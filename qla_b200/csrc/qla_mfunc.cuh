@@ -11,15 +11,15 @@
 //    stopping norm in double, FLT_EPSILON / DBL_EPSILON threshold):
 //    bit-identical to QLA_F3 and QLA_D3.
 //  exp: Cayley-Hamilton-reduced Taylor series with FP64 coefficients.  With
-//    B = A / 2^k (|B|_F <= 1) and B^3 = c2 B^2 + c1 B + c0 1, every power
-//    B^j / j! = q0 1 + q1 B + q2 B^2 where (q0,q1,q2) follow the recurrence
-//    q' = (q2 c0, q0 + q2 c1, q1 + q2 c2) / (j+1); summing the terms gives
-//    exp(B) = f0 1 + f1 B + f2 B^2 with no eigenvalues involved, so nearly
-//    degenerate spectra need no special case; then k squarings.  D3: all of
-//    it in FP64 (26 terms).  F3: only the coefficients in FP64 (16 terms);
-//    B^2, the assembly and the squarings in FP32.  The reference's F3/D3 use a
-//    rational approximation with scaling (M_eq_exp_M.c:302-367); agreement is
-//    checked against its FP64 (D3) result.
+//    B = A / 2^k (|B|_F <= 1) and B^3 = c2 B^2 + c1 B + c0 1, a polynomial in B
+//    is h0 1 + h1 B + h2 B^2, and B times it is h2 c0, h0 + h2 c1, h1 + h2 c2:
+//    Horner's scheme on the triple (h0, h1, h2) sums the series in twelve fused
+//    multiply-adds per term, with no eigenvalues involved, so nearly degenerate
+//    spectra need no special case; then k squarings.  D3: all of it in FP64 (21
+//    terms).  F3: only the coefficients in FP64 (16 terms); B^2, the assembly
+//    and the squarings in FP32.  The reference's F3/D3 use a rational
+//    approximation with scaling (M_eq_exp_M.c:302-367); agreement is checked
+//    against its FP64 (D3) result.
 #pragma once
 #include "qla_engine.cuh"
 
@@ -311,175 +311,106 @@ __device__ __forceinline__ Cx<T> det3_fast(const Cx<T> (&a)[9]) {
 }
 
 // ---------------------------------------------------------------------------
-// M_eq_exp_M: Cayley-Hamilton-reduced Taylor series (see header)
+// M_eq_exp_M: Cayley-Hamilton-reduced Taylor series (see header).  The kernel is
+// bound by the FP64 pipe.  (Summing the terms from the first up, with the powers
+// of B by the same recurrence, took 28 unfused operations per term instead of
+// 12: F3 on 24^3 x 48 sites 49 us, 31 so.)
+
+// 1/j! for j = 0 .. 20
+__device__ __constant__ const double kInvFact[21] = {
+    1.0, 1.0, 1.0 / 2.0, 1.0 / 6.0, 1.0 / 24.0, 1.0 / 120.0, 1.0 / 720.0, 1.0 / 5040.0, 1.0 / 40320.0, 1.0 / 362880.0,
+    1.0 / 3628800.0, 1.0 / 39916800.0, 1.0 / 479001600.0, 1.0 / 6227020800.0, 1.0 / 87178291200.0,
+    1.0 / 1307674368000.0, 1.0 / 20922789888000.0, 1.0 / 355687428096000.0, 1.0 / 6402373705728000.0,
+    1.0 / 121645100408832000.0, 1.0 / 2432902008176640000.0};
+
+// x + a b, fused
+__device__ __forceinline__ Cx<double> cfma(Cx<double> a, Cx<double> b, Cx<double> x) {
+  return Cx<double>{fma(a.re, b.re, fma(-a.im, b.im, x.re)), fma(a.re, b.im, fma(a.im, b.re, x.im))};
+}
+
+// f0, f1, f2 with sum_{j <= LAST} B^j / j! = f0 1 + f1 B + f2 B^2
+template <int LAST>
+__device__ __forceinline__ void exp_coefficients(const Cx<double> (&b)[9], Cx<double>& f0, Cx<double>& f1,
+                                                 Cx<double>& f2) {
+  const Cx<double> trb{b[0].re + b[4].re + b[8].re, b[0].im + b[4].im + b[8].im};
+  Cx<double> trb2{0.0, 0.0};  // tr B^2 = sum_ik b_ik b_ki
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    trb2 = cfma(b[i * 4], b[i * 4], trb2);
+#pragma unroll
+    for (int k = i + 1; k < 3; k++) {
+      const Cx<double> u = b[i * 3 + k], v = b[k * 3 + i];
+      const Cx<double> u2{2.0 * u.re, 2.0 * u.im};
+      trb2 = cfma(u2, v, trb2);
+    }
+  }
+  // B^3 = c2 B^2 + c1 B + c0 1  (Cayley-Hamilton)
+  const Cx<double> c2 = trb;
+  const Cx<double> c1{-0.5 * (trb.re * trb.re - trb.im * trb.im - trb2.re), -0.5 * (2.0 * trb.re * trb.im - trb2.im)};
+  const Cx<double> c0 = det3_fast(b);
+  f0 = Cx<double>{kInvFact[LAST - 2], 0.0};
+  f1 = Cx<double>{kInvFact[LAST - 1], 0.0};
+  f2 = Cx<double>{kInvFact[LAST], 0.0};
+#pragma unroll
+  for (int j = LAST - 3; j >= 0; j--) {
+    const Cx<double> n0 = cfma(f2, c0, Cx<double>{kInvFact[j], 0.0});
+    const Cx<double> n1 = cfma(f2, c1, f0);
+    f2 = cfma(f2, c2, f1);
+    f0 = n0;
+    f1 = n1;
+  }
+}
+
 template <typename R_>
 struct ExpOp {
   using R = R_;
   static constexpr int NIN = 1, N0 = 9, N1 = 0, N2 = 0, NOUT = 9, NACC = 0;
-  static constexpr int kTerms = 26;
-  // F3: 16 terms (the neglected tail is below 1/17! < 3e-15 of the result's
-  // scale when |B|_F <= 1)
-  static constexpr int kTermsF3 = 16;
-  __device__ static void apply(const SiteParams& p, const Cx<R> (&a)[9], const Cx<R> (&x1)[1],
-                               const Cx<R> (&x2)[1], Cx<R> (&r)[9]) {
-    if constexpr (sizeof(R) == 4)
-      apply_f3(a, r);
-    else
-      apply_d3(p, a, x1, x2, r);
-  }
-
-  // F3: FP64 only for the Cayley-Hamilton coefficients (the traces, the
-  // determinant and the Taylor recurrence on q0, q1, q2, computed from the
-  // exactly promoted float B); B^2, the assembly f0 + f1 B + f2 B^2 and the
-  // squarings in FP32 with fused multiply-adds.
-  __device__ static void apply_f3(const Cx<float> (&a)[9], Cx<float> (&r)[9]) {
+  // last power of the series: F3 B^15 (the neglected tail is below 1/16! =
+  // 5e-14 of the result's scale when |B|_F <= 1), D3 B^20 (2e-20)
+  static constexpr int kLast = sizeof(R) == 4 ? 15 : 20;
+  __device__ static void apply(const SiteParams&, const Cx<R> (&a)[9], const Cx<R> (&)[1], const Cx<R> (&)[1],
+                               Cx<R> (&r)[9]) {
     double fn = 0.0;
 #pragma unroll
     for (int k = 0; k < 9; k++) fn = fma((double)a[k].im, (double)a[k].im, fma((double)a[k].re, (double)a[k].re, fn));
     // B = A / 2^ks with |B|_F^2 <= 1: fn < 2^E, so ks = ceil(E / 2) suffices
     int ks = 0;
     if (fn > 1.0) {
-      int E;
-      frexp(fn, &E);
+      const int E = ((__double2hiint(fn) >> 20) & 0x7ff) - 1022;
       ks = (E + 1) >> 1;
       if (ks > 60) ks = 60;
     }
-    const float sc = ldexpf(1.0f, -ks);  // exact power of two
-    Cx<float> b[9];
-#pragma unroll
-    for (int k = 0; k < 9; k++) b[k] = Cx<float>{a[k].re * sc, a[k].im * sc};
-    // coefficients in FP64: tr B, tr B^2 = sum_ik b_ik b_ki, det B
+    const R sc = (R)__hiloint2double((1023 - ks) << 20, 0);  // 2^-ks, exact
+    Cx<R> b[9];
     Cx<double> bd[9];
 #pragma unroll
-    for (int k = 0; k < 9; k++) bd[k] = cd(b[k]);
-    const Cx<double> trb{bd[0].re + bd[4].re + bd[8].re, bd[0].im + bd[4].im + bd[8].im};
-    Cx<double> trb2{0.0, 0.0};
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-      for (int k = 0; k < 3; k++) {
-        const Cx<double> u = bd[i * 3 + k], v = bd[k * 3 + i];
-        trb2.re = fma(u.re, v.re, fma(-u.im, v.im, trb2.re));
-        trb2.im = fma(u.re, v.im, fma(u.im, v.re, trb2.im));
-      }
-    const Cx<double> c2 = trb;
-    const Cx<double> c1{-0.5 * (trb.re * trb.re - trb.im * trb.im - trb2.re),
-                        -0.5 * (2.0 * trb.re * trb.im - trb2.im)};
-    const Cx<double> c0 = det3_fast(bd);
-    Cx<double> q0{1.0, 0.0}, q1{0.0, 0.0}, q2{0.0, 0.0};
-    Cx<double> f0 = q0, f1 = q1, f2 = q2;
-#pragma unroll 3
-    for (int j = 1; j < kTermsF3; j++) {
-      const double inv = 1.0 / (double)j;
-      const Cx<double> n0 = cmul_fast(q2, c0);
-      Cx<double> n1 = cmul_fast(q2, c1);
-      Cx<double> n2 = cmul_fast(q2, c2);
-      n1.re += q0.re;
-      n1.im += q0.im;
-      n2.re += q1.re;
-      n2.im += q1.im;
-      q0 = Cx<double>{n0.re * inv, n0.im * inv};
-      q1 = Cx<double>{n1.re * inv, n1.im * inv};
-      q2 = Cx<double>{n2.re * inv, n2.im * inv};
-      f0.re += q0.re;
-      f0.im += q0.im;
-      f1.re += q1.re;
-      f1.im += q1.im;
-      f2.re += q2.re;
-      f2.im += q2.im;
+    for (int k = 0; k < 9; k++) {
+      b[k] = Cx<R>{a[k].re * sc, a[k].im * sc};
+      bd[k] = cd(b[k]);
     }
-    const Cx<float> g0{(float)f0.re, (float)f0.im}, g1{(float)f1.re, (float)f1.im}, g2{(float)f2.re, (float)f2.im};
-    // FP32: B^2, the assembly, the squarings
-    Cx<float> b2[9], e[9];
+    Cx<double> f0, f1, f2;
+    exp_coefficients<kLast>(bd, f0, f1, f2);
+    // B^2, the assembly and the squarings in the site precision
+    const Cx<R> g0{(R)f0.re, (R)f0.im}, g1{(R)f1.re, (R)f1.im}, g2{(R)f2.re, (R)f2.im};
+    Cx<R> b2[9];
     mat3_mul_fast(b2, b, b);
 #pragma unroll
     for (int k = 0; k < 9; k++) {
-      Cx<float> t = cmul_fast(g1, b[k]);
-      const Cx<float> u = cmul_fast(g2, b2[k]);
+      Cx<R> t = cmul_fast(g1, b[k]);
+      const Cx<R> u = cmul_fast(g2, b2[k]);
       t.re += u.re;
       t.im += u.im;
       if (k % 4 == 0) {
         t.re += g0.re;
         t.im += g0.im;
       }
-      e[k] = t;
+      r[k] = t;
     }
     for (int s = 0; s < ks; s++) {
-      mat3_mul_fast(b2, e, e);
+      mat3_mul_fast(b2, r, r);
 #pragma unroll
-      for (int k = 0; k < 9; k++) e[k] = b2[k];
+      for (int k = 0; k < 9; k++) r[k] = b2[k];
     }
-#pragma unroll
-    for (int k = 0; k < 9; k++) r[k] = e[k];
-  }
-
-  // D3: the whole evaluation in FP64
-  __device__ static void apply_d3(const SiteParams&, const Cx<R> (&a)[9], const Cx<R> (&)[1], const Cx<R> (&)[1],
-                                  Cx<R> (&r)[9]) {
-    Cx<double> b[9];
-#pragma unroll
-    for (int k = 0; k < 9; k++) b[k] = cd(a[k]);
-    double fn = 0.0;
-#pragma unroll
-    for (int k = 0; k < 9; k++) fn += b[k].re * b[k].re + b[k].im * b[k].im;
-    // scale by 2^-k so that |B|_F <= 1 (exact: a power of two)
-    int ks = 0;
-    if (fn > 1.0) {
-      ks = (int)ceil(0.5 * log2(fn));
-      if (ks > 60) ks = 60;
-      const double sc = ldexp(1.0, -ks);
-#pragma unroll
-      for (int k = 0; k < 9; k++) b[k] = Cx<double>{b[k].re * sc, b[k].im * sc};
-    }
-    Cx<double> b2[9];
-    mat3_mul(b2, b, b);
-    const Cx<double> trb{b[0].re + b[4].re + b[8].re, b[0].im + b[4].im + b[8].im};
-    const Cx<double> trb2{b2[0].re + b2[4].re + b2[8].re, b2[0].im + b2[4].im + b2[8].im};
-    const Cx<double> trb_sq = cmul(trb, trb);
-    // B^3 = c2 B^2 + c1 B + c0 1  (Cayley-Hamilton)
-    const Cx<double> c2 = trb;
-    const Cx<double> c1{-0.5 * (trb_sq.re - trb2.re), -0.5 * (trb_sq.im - trb2.im)};
-    const Cx<double> c0 = det3(b);
-    Cx<double> q0{1.0, 0.0}, q1{0.0, 0.0}, q2{0.0, 0.0};
-    Cx<double> f0 = q0, f1 = q1, f2 = q2;
-#pragma unroll 2
-    for (int j = 1; j < kTerms; j++) {
-      const double inv = 1.0 / (double)j;
-      const Cx<double> n0 = cmul(q2, c0);
-      Cx<double> n1 = cmul(q2, c1);
-      Cx<double> n2 = cmul(q2, c2);
-      n1.re += q0.re;
-      n1.im += q0.im;
-      n2.re += q1.re;
-      n2.im += q1.im;
-      q0 = Cx<double>{n0.re * inv, n0.im * inv};
-      q1 = Cx<double>{n1.re * inv, n1.im * inv};
-      q2 = Cx<double>{n2.re * inv, n2.im * inv};
-      f0.re += q0.re;
-      f0.im += q0.im;
-      f1.re += q1.re;
-      f1.im += q1.im;
-      f2.re += q2.re;
-      f2.im += q2.im;
-    }
-    Cx<double> e[9];
-#pragma unroll
-    for (int k = 0; k < 9; k++) {
-      const Cx<double> t1 = cmul(f1, b[k]);
-      const Cx<double> t2 = cmul(f2, b2[k]);
-      e[k] = Cx<double>{t1.re + t2.re, t1.im + t2.im};
-      if (k % 4 == 0) {
-        e[k].re += f0.re;
-        e[k].im += f0.im;
-      }
-    }
-    for (int s = 0; s < ks; s++) {
-      mat3_mul(b2, e, e);
-#pragma unroll
-      for (int k = 0; k < 9; k++) e[k] = b2[k];
-    }
-#pragma unroll
-    for (int k = 0; k < 9; k++) r[k] = cround<R>(e[k]);
   }
   __device__ static void accum(const SiteParams&, const Cx<R> (&)[9], const Cx<R> (&)[1], const Cx<R> (&)[1],
                                double*) {}

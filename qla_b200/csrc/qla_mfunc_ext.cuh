@@ -10,7 +10,7 @@
 //   sqrtPH, invsqrtPH         M_eq_sqrtPH_M.c:84-197, M_eq_invsqrtPH_M.c:84-201
 //   eigenvalsH, eigenvals     V_eq_eigenvalsH_M.c:106-166,
 //                             V_eq_eigenvals_M.c:127-186 (cubic roots)
-//   reunit (no counterpart)   u (u^+ u)^(-1/2) from the pieces above
+//   reunit (no counterpart)   u (u^+ u)^(-1/2) by invsqrtPH's closed form
 //
 // Precision.  a^-1 b uses only +, -, *, / and is evaluated in the site
 // precision with explicitly rounded operations: bit-identical to QLA_F3 and
@@ -27,6 +27,7 @@
 // may differ by an ulp, so D3 agrees with QLA_D3 to a few ulps away from
 // the templates' branch points.
 #pragma once
+#include "qla_launch.cuh"
 #include "qla_mfunc.cuh"
 #include "qla_ops.cuh"
 
@@ -262,6 +263,13 @@ struct LogOp {
   __device__ static void finish(const SiteParams&, const double*) {}
 };
 
+// (FP64 arithmetic: 770 us on the bulk-copy kernel, whose 288 threads leave 168
+// registers and spills, 686 us warp-cooperative; D3, 24^3 x 48)
+template <>
+struct ComputeBound<LogOp<double>> {
+  static constexpr bool value = true;
+};
+
 // ---------------------------------------------------------------------------
 // exp of a traceless anti-Hermitian i Q: eigenvalues of Q from
 // x^3 - p2/2 x - det = 0, exp(iQ) = f0 + f1 (iQ) + f2 (iQ)^2
@@ -488,21 +496,64 @@ struct SqrtPHOp {
 };
 
 // Unitarity reprojection r = u (u^+ u)^(-1/2), with no counterpart in the
-// reference: the composition QLA_D3_M_eq_Ma_times_M -> M_eq_invsqrtPH_M ->
-// M_eq_M_times_M evaluated in FP64 with those functions' operation order,
-// fused so that u is read once and r written once.
+// reference: the closed form of M_eq_invsqrtPH_M on t = u^+ u, in FP64, fused
+// so that u is read once and r written once.  The FP64 pipe bounds it, so t and
+// t^2 are formed as the Hermitian matrices they are (six elements, real
+// diagonals) and every product is fused with its sum: about 230 operations
+// beside the closed form, where the composition of M_eq_Ma_times_M,
+// M_eq_invsqrtPH_M and M_eq_M_times_M, each operation rounded, takes about 750.
+// Measured, F3 on 24^3 x 48 sites: 62 us as that composition,
+// 45 so (66 and 36 between events, after a cold start).
 template <typename R_>
 struct ReunitOp {
   using R = R_;
   static constexpr int NIN = 1, N0 = 9, N1 = 0, N2 = 0, NOUT = 9, NACC = 0;
+  // sum_k conj(a_ki) a_kj
+  __device__ __forceinline__ static Cx<double> column_dot(const Cx<double> (&a)[9], int i, int j) {
+    Cx<double> x{0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      const Cx<double> u = a[k * 3 + i], v = a[k * 3 + j];
+      x.re = fma(u.im, v.im, fma(u.re, v.re, x.re));
+      x.im = fma(-u.im, v.re, fma(u.re, v.im, x.im));
+    }
+    return x;
+  }
+  __device__ __forceinline__ static double n2(Cx<double> a) { return fma(a.im, a.im, a.re * a.re); }
   __device__ static void apply(const SiteParams&, const Cx<R> (&a)[9], const Cx<R> (&)[1], const Cx<R> (&)[1],
                                Cx<R> (&r)[9]) {
-    Cx<double> u[9], t[9], s[9];
+    Cx<double> u[9];
     promote9(u, a);
-    lmult_site<double, 3, 3, true, false>(EQ, false, u, u, t);   // u^+ u
-    sqrtph3_fp64<true>(s, t);                                     // (u^+ u)^(-1/2)
-    lmult_site<double, 3, 3, false, false>(EQ, false, u, s, t);  // u s
-    round_out(r, t);
+    // t = u^+ u: diagonal d0, d1, d2; t01, t02, t12 above it
+    const double d0 = column_dot(u, 0, 0).re, d1 = column_dot(u, 1, 1).re, d2 = column_dot(u, 2, 2).re;
+    const Cx<double> t01 = column_dot(u, 0, 1), t02 = column_dot(u, 0, 2), t12 = column_dot(u, 1, 2);
+    const double n01 = n2(t01), n02 = n2(t02), n12 = n2(t12);
+    // t^2: diagonal and upper elements
+    const double e0 = fma(d0, d0, n01 + n02), e1 = fma(d1, d1, n01 + n12), e2 = fma(d2, d2, n02 + n12);
+    const double s01 = d0 + d1, s02 = d0 + d2, s12 = d1 + d2;
+    const Cx<double> ct12{t12.re, -t12.im}, ct01{t01.re, -t01.im};
+    const Cx<double> q01 = cfma(t02, ct12, Cx<double>{s01 * t01.re, s01 * t01.im});
+    const Cx<double> q02 = cfma(t01, t12, Cx<double>{s02 * t02.re, s02 * t02.im});
+    const Cx<double> q12 = cfma(ct01, t02, Cx<double>{s12 * t12.re, s12 * t12.im});
+    const double tr = d0 + d1 + d2, p2 = e0 + e1 + e2;
+    // det t = d0 d1 d2 + 2 Re(t01 t12 conj(t02)) - d0 |t12|^2 - d1 |t02|^2 - d2 |t01|^2
+    const Cx<double> m = cfma(t01, t12, Cx<double>{0.0, 0.0});
+    const double re = fma(m.im, t02.im, m.re * t02.re);
+    const double det = fma(d0, fma(d1, d2, -n12), fma(2.0, re, fma(-d1, n02, -d2 * n01)));
+    double f0, f1, f2;
+    getfs_sqrtph<true>(f0, f1, f2, tr, p2, det);
+    // s = f0 + f1 t + f2 t^2, r = u s
+    const double h0 = fma(f2, e0, fma(f1, d0, f0)), h1 = fma(f2, e1, fma(f1, d1, f0)), h2 = fma(f2, e2, fma(f1, d2, f0));
+    auto mix = [&](Cx<double> t, Cx<double> q) { return Cx<double>{fma(f2, q.re, f1 * t.re), fma(f2, q.im, f1 * t.im)}; };
+    const Cx<double> h01 = mix(t01, q01), h02 = mix(t02, q02), h12 = mix(t12, q12);
+    const Cx<double> h10{h01.re, -h01.im}, h20{h02.re, -h02.im}, h21{h12.re, -h12.im};
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      const Cx<double> x = u[i * 3], y = u[i * 3 + 1], z = u[i * 3 + 2];
+      r[i * 3] = cround<R>(cfma(z, h20, cfma(y, h10, Cx<double>{x.re * h0, x.im * h0})));
+      r[i * 3 + 1] = cround<R>(cfma(z, h21, cfma(x, h01, Cx<double>{y.re * h1, y.im * h1})));
+      r[i * 3 + 2] = cround<R>(cfma(x, h02, cfma(y, h12, Cx<double>{z.re * h2, z.im * h2})));
+    }
   }
   __device__ static void accum(const SiteParams&, const Cx<R> (&)[9], const Cx<R> (&)[1], const Cx<R> (&)[1],
                                double*) {}
