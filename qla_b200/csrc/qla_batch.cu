@@ -357,6 +357,7 @@ __device__ __forceinline__ void fetch_tile(const BField& F, LaneStream& L, unsig
 // A warp's shared memory: [two stage barriers | field descriptor | index
 // tiles (fixed_bytes) | one or two stages].
 __global__ void __launch_bounds__(128, 4) batch_program_kernel(const BatchParams p) {
+  overlap_begin();
   extern __shared__ __align__(128) unsigned char smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned nw = blockDim.x >> 5;
@@ -392,7 +393,7 @@ __global__ void __launch_bounds__(128, 4) batch_program_kernel(const BatchParams
     }
     for (; g < gend && alive; f++) {
       const uint4* src = reinterpret_cast<const uint4*>(p.fields + f);
-      for (int k = lane; k < kDescWords; k += 32) desc[k] = __ldg(src + k);
+      for (int k = lane; k < kDescWords; k += 32) desc[k] = ld_in(src + k);
       __syncwarp();
       const long long ntf = (F.n + 31) / 32;  // tiles of this field (an empty field has none)
       const int ntail = (int)(F.n & 31);      // sites of a partial last tile
@@ -855,9 +856,8 @@ extern "C" QLAB_EXPORT int qlagpu_batch_run(void* handle) {
   p.stages = plan->stages;
   p.runs = plan->runs;
   p.err = device_error_word();
-  void* args[] = {&p};
-  if (cudaLaunchKernel(reinterpret_cast<const void*>(&batch_program_kernel), dim3((unsigned)plan->grid),
-                       dim3((unsigned)plan->threads), args, plan->smem, current_stream()) != cudaSuccess) {
+  if (launch_kernel(&batch_program_kernel, (unsigned)plan->grid, (unsigned)plan->threads, plan->smem, current_stream(),
+                    p) != cudaSuccess) {
     check_launch("qlagpu_batch_run");
     return QLAGPU_ERR_LAUNCH;
   }

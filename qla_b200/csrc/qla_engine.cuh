@@ -205,6 +205,7 @@ __global__ void __launch_bounds__(288) site_tma_kernel(const SiteParams p) {
   constexpr int OB = OP::NOUT * (int)sizeof(Cx<R>);
   constexpr int NA = ArrN<OP::NACC>::value;
   extern __shared__ __align__(128) unsigned char smem[];
+  overlap_begin();
   const int S = p.stages;
   const int NW = (blockDim.x >> 5) - 1;  // consumer warps
   const int T = NW * 32;                 // sites per tile
@@ -475,6 +476,7 @@ __global__ void __launch_bounds__(128, coop_min_blocks<OP>()) site_coop_kernel(c
   using L = CoopLayout<OP>;
   constexpr int NA = ArrN<OP::NACC>::value, C = (int)sizeof(Cx<R>);
   extern __shared__ __align__(128) unsigned char smem[];
+  overlap_begin();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   unsigned char* sl = smem + (size_t)warp * L::warp_bytes;
   DD dacc[NA];
@@ -538,6 +540,7 @@ __global__ void __launch_bounds__(128, coop_min_blocks<OP>()) site_coop_kernel(c
 // One site per thread, for the allocation-free entry point's unaligned calls.
 template <class OP>
 __global__ void __launch_bounds__(256) site_direct_kernel(const SiteParams p) {
+  overlap_begin();
   constexpr int NA = ArrN<OP::NACC>::value;
   DD dacc[NA];
 #pragma unroll

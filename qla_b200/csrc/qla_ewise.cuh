@@ -145,6 +145,7 @@ __device__ __forceinline__ Cx<R> ew_apply(int eqop, Cx<R> x, Cx<R> s, Cx<R> b, C
 
 template <typename R, int NE, int SHAPE, int PERM, int SCAL, bool SREAL>
 __global__ void __launch_bounds__(256) ew_kernel(const EwParams p) {
+  overlap_begin();
   constexpr bool TWO = SHAPE == EW_PLUS || SHAPE == EW_MINUS || SHAPE >= EW_RT_PLUS;
   const long long total = p.n * NE;
   const bool load = (p.eqop == PEQ || p.eqop == MEQ);
@@ -191,6 +192,7 @@ __global__ void __launch_bounds__(256) ew_kernel(const EwParams p) {
 // ew_apply, so results are identical.
 template <typename R, int NE, int SHAPE, int SCAL, bool SREAL>
 __global__ void __launch_bounds__(256) ew_flat_kernel(const EwParams p, long long nelem) {
+  overlap_begin();
   constexpr bool TWO = SHAPE == EW_PLUS || SHAPE == EW_MINUS || SHAPE >= EW_RT_PLUS;
   constexpr int CPV = 16 / (int)sizeof(Cx<R>);  // complex numbers per 16-B vector
   constexpr int CPT = 2 * CPV;                   // per thread and step
@@ -230,11 +232,11 @@ __global__ void __launch_bounds__(256) ew_flat_kernel(const EwParams p, long lon
     for (int h = 0; h < 2; h++) {
       const long long q = g0 + h * CPV;
       if constexpr (sizeof(R) == 4) {
-        const float4 u = __ldg(reinterpret_cast<const float4*>(B + q));
+        const float4 u = ld_in(reinterpret_cast<const float4*>(B + q));
         b[2 * h] = Cx<R>{u.x, u.y};
         b[2 * h + 1] = Cx<R>{u.z, u.w};
         if constexpr (TWO) {
-          const float4 w = __ldg(reinterpret_cast<const float4*>(C + q));
+          const float4 w = ld_in(reinterpret_cast<const float4*>(C + q));
           c[2 * h] = Cx<R>{w.x, w.y};
           c[2 * h + 1] = Cx<R>{w.z, w.w};
         }
@@ -244,10 +246,10 @@ __global__ void __launch_bounds__(256) ew_flat_kernel(const EwParams p, long lon
           x[2 * h + 1] = Cx<R>{o.z, o.w};
         }
       } else {
-        const double2 u = __ldg(reinterpret_cast<const double2*>(B + q));
+        const double2 u = ld_in(reinterpret_cast<const double2*>(B + q));
         b[h] = Cx<R>{u.x, u.y};
         if constexpr (TWO) {
-          const double2 w = __ldg(reinterpret_cast<const double2*>(C + q));
+          const double2 w = ld_in(reinterpret_cast<const double2*>(C + q));
           c[h] = Cx<R>{w.x, w.y};
         }
         if (load) {
@@ -320,11 +322,11 @@ inline void api_ew(const char* kid, void* r, const void* scal, Opnd s, Opnd b, O
     constexpr int CPT = 2 * (16 / (int)sizeof(Cx<R>));
     long long grid = (total / CPT + 255) / 256;
     if (grid > cap) grid = cap;
-    ew_flat_kernel<R, NE, SHAPE, SCAL, SREAL><<<(unsigned)(grid < 1 ? 1 : grid), 256, 0, current_stream()>>>(p, total);
+    launch_kernel(ew_flat_kernel<R, NE, SHAPE, SCAL, SREAL>, (unsigned)(grid < 1 ? 1 : grid), 256, 0, current_stream(), p, total);
   } else {
     long long grid = (total + 255) / 256;
     if (grid > cap) grid = cap;
-    ew_kernel<R, NE, SHAPE, PERM, SCAL, SREAL><<<(unsigned)(grid < 1 ? 1 : grid), 256, 0, current_stream()>>>(p);
+    launch_kernel(ew_kernel<R, NE, SHAPE, PERM, SCAL, SREAL>, (unsigned)(grid < 1 ? 1 : grid), 256, 0, current_stream(), p);
   }
   check_launch(kid);
 }
@@ -352,6 +354,7 @@ struct OuterOp {
 
 template <typename R>
 __global__ void __launch_bounds__(256) outer_kernel(const EwParams p) {
+  overlap_begin();
   const long long total = p.n * 9;
   const bool load = (p.eqop == PEQ || p.eqop == MEQ);
   for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < total;
@@ -390,7 +393,7 @@ inline void api_outer(const char* kid, void* r, Opnd a, Opnd b, const int* gang,
   long long grid = ((long long)n * 9 + 255) / 256;
   const long long cap = (long long)device_sm_count() * 16;
   if (grid > cap) grid = cap;
-  outer_kernel<R><<<(unsigned)(grid < 1 ? 1 : grid), 256, 0, current_stream()>>>(p);
+  launch_kernel(outer_kernel<R>, (unsigned)(grid < 1 ? 1 : grid), 256, 0, current_stream(), p);
   check_launch(kid);
 }
 
@@ -462,6 +465,7 @@ __device__ __forceinline__ void ldot_store(void* out, long long k, int eqop, dou
 // one thread per site, records read where they are (gang or pointer forms)
 template <typename R, int KIND>
 __global__ void __launch_bounds__(256) ldot_kernel(const EwParams p, int ne, int blk) {
+  overlap_begin();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < p.n;
        i += (long long)gridDim.x * blockDim.x) {
     const long long k = p.gang ? (long long)p.gang[i] : i;
@@ -491,6 +495,7 @@ __global__ void __launch_bounds__(256) ldot_kernel(const EwParams p, int ne, int
 __host__ __device__ inline unsigned ldot_slot(unsigned rb) { return (rb % 128u == 0u) ? rb + 16u : rb; }
 template <typename R, int KIND>
 __global__ void __launch_bounds__(128) ldot_tile_kernel(const EwParams p, int ne, int blk, int bulk, unsigned* err) {
+  overlap_begin();
   extern __shared__ __align__(128) unsigned char ldsm[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   constexpr int NOP = KIND == LD_NORM2 ? 1 : 2;
@@ -609,11 +614,11 @@ inline void run_ldot(const char* kid, int ne, int blk, void* r, Opnd a, Opnd b, 
     // unevenly: norm2_D 20 us, 13 so)
     const long long grid = ((long long)n + 32 * nw - 1) / (32 * nw);
     const int bulk = aligned16(a.base) && (KIND == LD_NORM2 || aligned16(b.base)) ? 1 : 0;
-    ldot_tile_kernel<R, KIND><<<(unsigned)grid, 32 * nw, smem, current_stream()>>>(p, ne, blk, bulk, device_error_word());
+    launch_kernel(ldot_tile_kernel<R, KIND>, (unsigned)grid, 32 * nw, smem, current_stream(), p, ne, blk, bulk, device_error_word());
   } else {
     long long grid = ((long long)n + 255) / 256;
     if (grid > (long long)sms * 16) grid = (long long)sms * 16;
-    ldot_kernel<R, KIND><<<(unsigned)(grid < 1 ? 1 : grid), 256, 0, current_stream()>>>(p, ne, blk);
+    launch_kernel(ldot_kernel<R, KIND>, (unsigned)(grid < 1 ? 1 : grid), 256, 0, current_stream(), p, ne, blk);
   }
   check_launch(kid);
 }

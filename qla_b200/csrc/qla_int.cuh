@@ -79,7 +79,8 @@ __device__ __forceinline__ int int_fetch(const Opnd& o, long long k) {
 }
 
 __global__ void __launch_bounds__(256) int_kernel(const IntParams p) {
-  const int s = p.sptr ? __ldg(p.sptr) : p.sval;
+  overlap_begin();
+  const int s = p.sptr ? ld_in(p.sptr) : p.sval;
   const bool rd = (p.eqop == PEQ || p.eqop == MEQ || p.code == IC_MASK);
   const long long stride = (long long)gridDim.x * blockDim.x;
   if (p.vec) {
@@ -87,9 +88,9 @@ __global__ void __launch_bounds__(256) int_kernel(const IntParams p) {
     const long long n4 = p.n / 4;
     for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += stride) {
       int4 av = make_int4(0, 0, 0, 0), bv = av, cv = av, rv = av;
-      if (p.nin > 0) av = __ldg(static_cast<const int4*>(p.in[0].base) + q);
-      if (p.nin > 1) bv = __ldg(static_cast<const int4*>(p.in[1].base) + q);
-      if (p.nin > 2) cv = __ldg(static_cast<const int4*>(p.in[2].base) + q);
+      if (p.nin > 0) av = ld_in(static_cast<const int4*>(p.in[0].base) + q);
+      if (p.nin > 1) bv = ld_in(static_cast<const int4*>(p.in[1].base) + q);
+      if (p.nin > 2) cv = ld_in(static_cast<const int4*>(p.in[2].base) + q);
       if (rd) rv = reinterpret_cast<const int4*>(p.out)[q];
       rv.x = int_apply(p.code, p.eqop, rv.x, av.x, bv.x, cv.x, s);
       rv.y = int_apply(p.code, p.eqop, rv.y, av.y, bv.y, cv.y, s);
@@ -151,7 +152,7 @@ inline void api_int(const char* kid, int code, int eqop, int* r, const int* s, O
   const long long cap = (long long)device_sm_count() * 16;
   if (want > cap) want = cap;
   if (want < 1) want = 1;
-  int_kernel<<<(unsigned)want, threads, 0, current_stream()>>>(p);
+  launch_kernel(int_kernel, (unsigned)want, threads, 0, current_stream(), p);
   check_launch(kid);
 }
 

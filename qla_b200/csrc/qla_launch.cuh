@@ -19,6 +19,30 @@ struct LaunchShape {
   int stages;
 };
 
+// Every kernel goes out through here, with programmatic stream serialisation:
+// its blocks come onto the SMs as soon as the blocks of the kernel before have
+// ended, and wait there (overlap_begin) until that kernel's writes are visible,
+// so a call does not cost the stream the whole launch latency.  Order and
+// results are a plain launch's; inside a captured graph the edge is a
+// programmatic one.  Measured: the 24 calls of a Wilson hop on 8^4 sites 114 us
+// in plain launches, 93 so; on 32^3 x 64 1472 / 1420; eight fused terms on its
+// even sites 875 / 857.
+template <class... P, class... A>
+inline cudaError_t launch_kernel(void (*fn)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st,
+                                 A&&... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, fn, P(args)...);
+}
+
 // shared memory of one block of the pipelined kernel
 inline size_t tma_smem_bytes(int threads, int stages, unsigned stage_bytes, unsigned out_bytes) {
   return 256 + (size_t)stages * stage_bytes + 2 * (size_t)threads * out_bytes;
@@ -149,8 +173,7 @@ struct SiteLauncher {
       const long long cap = (long long)launch_blocks_per_sm(fn, 32 * nw, smem) * sms;
       if (grid > cap) grid = cap;
       if (reduce && grid > rs->max_blocks) grid = rs->max_blocks;
-      void* args[] = {&p};
-      if (cudaLaunchKernel(fn, dim3((unsigned)grid), dim3(32u * nw), args, smem, st) != cudaSuccess) {
+      if (launch_kernel(&site_coop_kernel<OP>, (unsigned)grid, 32u * nw, smem, st, p) != cudaSuccess) {
         check_launch(kernel_id);
         return;
       }
@@ -212,9 +235,8 @@ struct SiteLauncher {
       if (grid > p.ntiles) grid = p.ntiles;
       if (grid < 1) grid = 1;
       if (reduce && grid > rs->max_blocks) grid = rs->max_blocks;
-      void* args[] = {&p};
       // T consumer threads + one producer warp
-      if (cudaLaunchKernel(fn, dim3((unsigned)grid), dim3((unsigned)T + 32u), args, smem, st) != cudaSuccess) {
+      if (launch_kernel(&site_tma_kernel<OP>, (unsigned)grid, (unsigned)T + 32u, smem, st, p) != cudaSuccess) {
         check_launch(kernel_id);
         return;
       }

@@ -151,6 +151,7 @@ __device__ void exp_pade(Mat<R, NC>& r, const Mat<R, NC>& a) {
       m_eq_m_times_m(t, va, pb);
       va = t;
     }
+    if (s == 1u) break;  // the last square is not used
     m_eq_m_times_m(t, pb, pb);
     pb = t;
   }

@@ -59,6 +59,7 @@ __device__ __forceinline__ void multi_site_direct(const MultiParams& p, long lon
 
 template <typename R, bool ADJ>
 __global__ void __launch_bounds__(256) multi_direct_kernel(const MultiParams p) {
+  overlap_begin();
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < p.n; i += stride)
     multi_site_direct<R, ADJ>(p, p.gang ? (long long)p.gang[i] : i);
@@ -68,6 +69,7 @@ __global__ void __launch_bounds__(256) multi_direct_kernel(const MultiParams p) 
 // operand tiles per stage
 template <typename R, bool ADJ>
 __global__ void __launch_bounds__(288) multi_tma_kernel(const MultiParams p) {
+  overlap_begin();
   constexpr int RM = 9 * (int)sizeof(Cx<R>), RV = 3 * (int)sizeof(Cx<R>);
   extern __shared__ __align__(128) unsigned char smem[];
   const int S = p.stages;
@@ -244,7 +246,7 @@ inline void api_multi(const char* kid, void* r, const void* a, bool pa, const vo
     if (direct) {
       long long grid = ((long long)n + 255) / 256;
       if (grid > (long long)sms * 8) grid = (long long)sms * 8;
-      multi_direct_kernel<R, ADJ><<<(unsigned)(grid < 1 ? 1 : grid), 256, 0, st>>>(p);
+      launch_kernel(multi_direct_kernel<R, ADJ>, (unsigned)(grid < 1 ? 1 : grid), 256, 0, st, p);
     } else {
       const unsigned bps = (unsigned)p.nd * ((pa ? 8u : RM) + (pb ? 8u : RV)) + (p.out_read ? RV : 0u);
       LaunchShape sh = default_shape(bps, RV);
@@ -273,8 +275,7 @@ inline void api_multi(const char* kid, void* r, const void* a, bool pa, const vo
       long long grid = (long long)nb * sms;
       if (grid > p.ntiles) grid = p.ntiles;
       if (grid < 1) grid = 1;
-      void* args[] = {&p};
-      if (cudaLaunchKernel(fn, dim3((unsigned)grid), dim3((unsigned)T + 32u), args, smem, st) != cudaSuccess) {
+      if (launch_kernel(&multi_tma_kernel<R, ADJ>, (unsigned)grid, (unsigned)T + 32u, smem, st, p) != cudaSuccess) {
         check_launch(kid);
         return;
       }

@@ -105,6 +105,7 @@ inline bool nc_ok(const char* kid, int nc) {
 // element-wise families (qla_ewise.cuh api_ew with run-time ne / perm)
 template <typename R, int SHAPE, int SCAL, bool SREAL>
 __global__ void __launch_bounds__(256) ewn_kernel(const EwParams p, const NcDims d) {
+  overlap_begin();
   constexpr bool TWO = SHAPE == EW_PLUS || SHAPE == EW_MINUS || SHAPE >= EW_RT_PLUS;
   const bool load = (p.eqop == PEQ || p.eqop == MEQ);
   const int ne = d.ne;
@@ -167,13 +168,14 @@ inline void api_ew_n(const char* kid, int nc, int ne, int perm, void* r, const v
       p.sim = (double)static_cast<const Cx<R>*>(scal)->im;
     }
   }
-  ewn_kernel<R, SHAPE, SCAL, SREAL><<<nc_grid((long long)n * ne), 256, 0, current_stream()>>>(p, nc_dims(nc, ne, perm));
+  launch_kernel(ewn_kernel<R, SHAPE, SCAL, SREAL>, nc_grid((long long)n * ne), 256, 0, current_stream(), p, nc_dims(nc, ne, perm));
   check_launch(kid);
 }
 
 // outer product M (eqop) a b^+ of two nc-vectors
 template <typename R>
 __global__ void __launch_bounds__(256) outern_kernel(const EwParams p, int nc) {
+  overlap_begin();
   const int m = nc * nc;
   const float inv = 1.0f / (float)nc;
   const bool load = (p.eqop == PEQ || p.eqop == MEQ);
@@ -203,7 +205,7 @@ inline void api_outer_n(const char* kid, int nc, void* r, Opnd a, Opnd b, const 
   p.gang = gang;
   p.n = n;
   p.eqop = eqop;
-  outern_kernel<R><<<nc_grid((long long)n * nc * nc), 256, 0, current_stream()>>>(p, nc);
+  launch_kernel(outern_kernel<R>, nc_grid((long long)n * nc * nc), 256, 0, current_stream(), p, nc);
   check_launch(kid);
 }
 
@@ -268,6 +270,7 @@ __device__ __forceinline__ int sfn_ops(const SfnParams& p, int KIND) {
 
 template <typename R, int KIND>
 __global__ void __launch_bounds__(256) sfn_kernel(const SfnParams p) {
+  overlap_begin();
   const int ops = sfn_ops(p, KIND);
   const int nc = p.nc;
   const float inv_nc = 1.0f / (float)nc, inv_4nc = 1.0f / (float)(4 * nc);
@@ -386,7 +389,7 @@ inline bool sfn_prep(const char* kid, SfnParams& p, int nc, void* r, Opnd a, con
 
 template <typename R, int KIND>
 inline void sfn_launch(const char* kid, const SfnParams& p, long long ops) {
-  sfn_kernel<R, KIND><<<nc_grid(p.n * ops), 256, 0, current_stream()>>>(p);
+  launch_kernel(sfn_kernel<R, KIND>, nc_grid(p.n * ops), 256, 0, current_stream(), p);
   check_launch(kid);
 }
 
@@ -535,6 +538,7 @@ inline void api_antiherm_n(const char* kid, int nc, void* r, Opnd a, const int* 
 // global reductions of P and of the adjoint forms, one thread per site
 template <typename R, int KIND, typename OUT>
 __global__ void __launch_bounds__(256) gdotn_kernel(const EwParams p, const SiteParams rp, const NcDims d) {
+  overlap_begin();
   using FIN = GDotFinish<KIND, OUT>;
   DD acc[ArrN<FIN::NACC>::value];
 #pragma unroll
@@ -557,6 +561,7 @@ __global__ void __launch_bounds__(256) gdotn_kernel(const EwParams p, const Site
 // unpermuted forms need no element positions and take its grouped sums)
 template <typename R, int KIND, typename OUT>
 __global__ void __launch_bounds__(256, 4) gdotn_flat_kernel(const EwParams p, const SiteParams rp, const NcDims d) {
+  overlap_begin();
   using FIN = GDotFinish<KIND, OUT>;
   if constexpr (KIND == LD_DOT || KIND == LD_REDOT || KIND == LD_NORM2) {
     DD acc[ArrN<FIN::NACC>::value];
@@ -657,9 +662,9 @@ inline void api_gdot_n(const char* kid, int nc, int ne, int perm, void* r, Opnd 
   if (grid > cap) grid = cap;
   if (grid > rs->max_blocks) grid = rs->max_blocks;
   if (flat)
-    gdotn_flat_kernel<R, KIND, OUT><<<(unsigned)(grid < 1 ? 1 : grid), 256, 0, st>>>(p, rp, nc_dims(nc, ne, perm));
+    launch_kernel(gdotn_flat_kernel<R, KIND, OUT>, (unsigned)(grid < 1 ? 1 : grid), 256, 0, st, p, rp, nc_dims(nc, ne, perm));
   else
-    gdotn_kernel<R, KIND, OUT><<<(unsigned)(grid < 1 ? 1 : grid), 256, 0, st>>>(p, rp, nc_dims(nc, ne, perm));
+    launch_kernel(gdotn_kernel<R, KIND, OUT>, (unsigned)(grid < 1 ? 1 : grid), 256, 0, st, p, rp, nc_dims(nc, ne, perm));
   if (!check_launch(kid)) return;
   if (!dev_out) {
     if (cudaMemcpyAsync(r, rs->result, rbytes, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
@@ -680,6 +685,7 @@ constexpr int GSUM_Q = 8;
 
 template <typename R, bool WIDE>
 __global__ void __launch_bounds__(1024, WIDE ? 1 : 2) gsumn_kernel(const EwParams p, int NR, DD* partials, int flat) {
+  overlap_begin();
   extern __shared__ __align__(16) unsigned char gsnm[];
   DD* red = reinterpret_cast<DD*>(gsnm);
   const int BT = blockDim.x;
@@ -784,11 +790,11 @@ inline void api_gsum_n(const char* kid, int nc, int ne, void* r, Opnd a, const i
   const int flat = (gang == nullptr && a.mode == OM_CONTIG) ? 1 : 0;
   const size_t smem = wide ? 0 : (size_t)BT * sizeof(DD);
   if (wide)
-    gsumn_kernel<R, true><<<(unsigned)grid, BT, smem, st>>>(p, NR, rs->partials, flat);
+    launch_kernel(gsumn_kernel<R, true>, (unsigned)grid, BT, smem, st, p, NR, rs->partials, flat);
   else
-    gsumn_kernel<R, false><<<(unsigned)grid, BT, smem, st>>>(p, NR, rs->partials, flat);
+    launch_kernel(gsumn_kernel<R, false>, (unsigned)grid, BT, smem, st, p, NR, rs->partials, flat);
   if (!check_launch(kid)) return;
-  gsum_fold_kernel<OUT><<<NR, GS_FOLD, 0, st>>>(rs->partials, (int)grid, NR, res);
+  launch_kernel(gsum_fold_kernel<OUT>, NR, GS_FOLD, 0, st, rs->partials, (int)grid, NR, res);
   if (!check_launch(kid)) return;
   if (!dev_out) {
     if (cudaMemcpyAsync(r, res, rbytes, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
@@ -800,6 +806,7 @@ inline void api_gsum_n(const char* kid, int nc, int ne, void* r, Opnd a, const i
 // precision conversions with run-time record length
 template <typename RIN, typename ROUT>
 __global__ void __launch_bounds__(256) convertn_kernel(const EwParams p, int NR) {
+  overlap_begin();
   for (SiteElemWalk w(NR); w.i < p.n; w.next(NR)) {
     const long long k = p.gang ? (long long)p.gang[w.i] : w.i;
     const RIN* src = (p.b.mode == OM_PTR) ? static_cast<const RIN*>(p.b.ptrs[k]) : static_cast<const RIN*>(p.b.base) + k * NR;
@@ -820,7 +827,7 @@ inline void api_convert_n(const char* kid, int nc, int ne, void* r, Opnd a, cons
   p.b = a;
   p.gang = gang;
   p.n = n;
-  convertn_kernel<RIN, ROUT><<<nc_grid((long long)n * 2 * ne), 256, 0, current_stream()>>>(p, 2 * ne);
+  launch_kernel(convertn_kernel<RIN, ROUT>, nc_grid((long long)n * 2 * ne), 256, 0, current_stream(), p, 2 * ne);
   check_launch(kid);
 }
 
@@ -832,6 +839,7 @@ inline void api_convert_n(const char* kid, int nc, int ne, void* r, Opnd a, cons
 // e = ((ic*4 + is)*nc + jc)*4 + js for P, ic*nc + jc for the trace's M.
 template <typename R, int KIND, bool CA, bool CB>
 __global__ void __launch_bounds__(256) propn_kernel(const EwParams p, int nc) {
+  overlap_begin();
   const int nm = nc * nc, np = 16 * nc * nc;
   const int nel = (KIND == PK_TRACE) ? nm : np;
   const int ra = (KIND == PK_MP) ? nm : np, rb = (KIND == PK_PM) ? nm : np;
@@ -886,7 +894,7 @@ inline void api_prop_n(const char* kid, int nc, void* r, Opnd a, Opnd b, const i
   p.n = n;
   p.eqop = eqop;
   const long long nel = (KIND == PK_TRACE) ? (long long)nc * nc : 16LL * nc * nc;
-  propn_kernel<R, KIND, CA, CB><<<nc_grid((long long)n * nel), 256, 0, current_stream()>>>(p, nc);
+  launch_kernel(propn_kernel<R, KIND, CA, CB>, nc_grid((long long)n * nel), 256, 0, current_stream(), p, nc);
   check_launch(kid);
 }
 
@@ -905,6 +913,7 @@ struct MultiNParams {
 
 template <typename R, bool ADJ>
 __global__ void __launch_bounds__(256) multin_kernel(const MultiNParams p) {
+  overlap_begin();
   const int nc = p.nc;
   for (SiteElemWalk w(nc); w.i < p.n; w.next(nc)) {
     const long long k = p.gang ? (long long)p.gang[w.i] : w.i;
@@ -954,7 +963,7 @@ inline void api_multi_n(const char* kid, int nc, void* r, const void* a, bool pa
       p.a[d] = pa ? op_ptr(static_cast<const void* const*>(ad)) : op_contig(ad);
       p.b[d] = pb ? op_ptr(static_cast<const void* const*>(bd)) : op_contig(bd);
     }
-    multin_kernel<R, ADJ><<<nc_grid((long long)n * nc), 256, 0, current_stream()>>>(p);
+    launch_kernel(multin_kernel<R, ADJ>, nc_grid((long long)n * nc), 256, 0, current_stream(), p);
     if (!check_launch(kid)) return;
   }
 }

@@ -298,7 +298,7 @@ struct SpprojDOp {
 // qla_complex.h:258-265 (scalar read once as `at = *a`).
 template <typename R>
 __device__ __forceinline__ R scalar_arg(const SiteParams& p) {
-  if (p.sptr) return __ldg(static_cast<const R*>(p.sptr));
+  if (p.sptr) return ld_in(static_cast<const R*>(p.sptr));
   return static_cast<R>(p.sval);
 }
 

@@ -194,12 +194,12 @@ __device__ __forceinline__ void ld2(Cx<R> (&v)[2], const Opnd& o, long long k, i
   if (vec) {
     const Cx<R>* base = static_cast<const Cx<R>*>(o.base) + k * rec + e;
     if constexpr (sizeof(R) == 4) {
-      const float4 u = __ldg(reinterpret_cast<const float4*>(base));
+      const float4 u = ld_in(reinterpret_cast<const float4*>(base));
       v[0] = Cx<R>{u.x, u.y};
       v[1] = Cx<R>{u.z, u.w};
     } else {
       const double2* q = reinterpret_cast<const double2*>(base);
-      const double2 u = __ldg(q), w = __ldg(q + 1);
+      const double2 u = ld_in(q), w = ld_in(q + 1);
       v[0] = Cx<R>{u.x, u.y};
       v[1] = Cx<R>{w.x, w.y};
     }
@@ -254,6 +254,7 @@ __device__ __forceinline__ void init2(Cx<R> (&x)[2], const Cx<R>* q, bool load, 
 // 2jh..2jh+1) for ic = 0..2
 template <typename R, bool CA, bool CB>
 __global__ void __launch_bounds__(256) prop_mp_kernel(const PropParams p) {
+  overlap_begin();
   const long long total = p.n * 24;
   const bool minus = (p.eqop == MEQ || p.eqop == EQM);
   const bool load = (p.eqop == PEQ || p.eqop == MEQ);
@@ -311,6 +312,7 @@ __global__ void __launch_bounds__(256) prop_mp_kernel(const PropParams p) {
 // 2jh..2jh+1) for jc = 0..2
 template <typename R, bool CA, bool CB>
 __global__ void __launch_bounds__(256) prop_pm_kernel(const PropParams p) {
+  overlap_begin();
   const long long total = p.n * 24;
   const bool minus = (p.eqop == MEQ || p.eqop == EQM);
   const bool load = (p.eqop == PEQ || p.eqop == MEQ);
@@ -355,6 +357,7 @@ __global__ void __launch_bounds__(256) prop_pm_kernel(const PropParams p) {
 // registers low enough for two blocks per SM.
 template <typename R, bool CA, bool CB>
 __global__ void __launch_bounds__(256) prop_pp_kernel(const PropParams p) {
+  overlap_begin();
   constexpr int JW = sizeof(R) == 4 ? 2 : 1;  // spin components per thread
   constexpr int TPS = 12 / JW;                 // threads per site
   const long long total = p.n * TPS;
@@ -510,6 +513,7 @@ constexpr int prop_tma_tps() {
 template <typename R, int KIND, bool CA, bool CB, int SPB, int MINB>
 __global__ void __launch_bounds__(prop_tma_tps<R, KIND>() * SPB + 32, MINB)
     prop_tma_kernel(const PropParams p, long long ntiles) {
+  overlap_begin();
   extern __shared__ __align__(128) unsigned char ptm[];
   constexpr int TPS = prop_tma_tps<R, KIND>();
   constexpr int NCT = TPS * SPB;  // consumer threads
@@ -896,6 +900,7 @@ inline int prop_blocks_per_sm(const void* fn, int threads, size_t smem) {
 // the spin trace: one thread per output element (9 per site)
 template <typename R>
 __global__ void __launch_bounds__(256) prop_trace_kernel(const PropParams p) {
+  overlap_begin();
   const long long total = p.n * 9;
   const bool minus = (p.eqop == MEQ || p.eqop == EQM);
   const bool load = (p.eqop == PEQ || p.eqop == MEQ);
@@ -951,15 +956,15 @@ inline void api_prop(const char* kid, void* r, Opnd a, Opnd b, const int* gang, 
   const bool contig =
       gang == nullptr && a.mode == OM_CONTIG && b.mode == OM_CONTIG && p.vec_a && p.vec_b && p.vec_out;
   if constexpr (KIND == PK_TRACE) {
-    prop_trace_kernel<R><<<gr, 256, 0, st>>>(p);
+    launch_kernel(prop_trace_kernel<R>, gr, 256, 0, st, p);
   } else if (!contig) {
     // gang, pointer or unaligned operands: the direct kernels
     if constexpr (KIND == PK_MP)
-      prop_mp_kernel<R, CA, CB><<<gr, 256, 0, st>>>(p);
+      launch_kernel(prop_mp_kernel<R, CA, CB>, gr, 256, 0, st, p);
     else if constexpr (KIND == PK_PM)
-      prop_pm_kernel<R, CA, CB><<<gr, 256, 0, st>>>(p);
+      launch_kernel(prop_pm_kernel<R, CA, CB>, gr, 256, 0, st, p);
     else
-      prop_pp_kernel<R, CA, CB><<<gr, 256, 0, st>>>(p);
+      launch_kernel(prop_pp_kernel<R, CA, CB>, gr, 256, 0, st, p);
   } else {
     // bulk-copy pipeline, tiles of 8 sites, 96 consumer threads + one
     // producer warp per block.  P * P: F3 three stages (57 KB), four blocks
@@ -990,7 +995,7 @@ inline void api_prop(const char* kid, void* r, Opnd a, Opnd b, const int* gang, 
       const int nb = prop_blocks_per_sm(fn, NT, smem);
       long long blocks = (long long)(nb < CAP ? nb : CAP) * device_sm_count();
       if (blocks > ntiles) blocks = ntiles;
-      prop_tma_kernel<R, KIND, CA, CB, SPB, MINB><<<(unsigned)blocks, NT, smem, st>>>(p, ntiles);
+      launch_kernel(prop_tma_kernel<R, KIND, CA, CB, SPB, MINB>, (unsigned)blocks, NT, smem, st, p, ntiles);
     }
     if constexpr (!PP) {
       const long long done = ntiles * SPB;
@@ -1002,9 +1007,9 @@ inline void api_prop(const char* kid, void* r, Opnd a, Opnd b, const int* gang, 
         t.out = static_cast<Cx<R>*>(r) + done * 144;
         t.n = n - done;
         if constexpr (KIND == PK_MP)
-          prop_mp_kernel<R, CA, CB><<<1, 256, 0, st>>>(t);
+          launch_kernel(prop_mp_kernel<R, CA, CB>, 1, 256, 0, st, t);
         else
-          prop_pm_kernel<R, CA, CB><<<1, 256, 0, st>>>(t);
+          launch_kernel(prop_pm_kernel<R, CA, CB>, 1, 256, 0, st, t);
       }
     }
   }

@@ -375,6 +375,7 @@ __device__ __forceinline__ void rng_load_table(LogEntry* table) {
 // states are scattered (gang index, pointers)
 template <typename R, int MODE>
 __global__ void __launch_bounds__(128) rng_fill_kernel(const RngParams p) {
+  overlap_begin();
   __shared__ __align__(16) LogEntry table[kRngTable];
   rng_load_table(table);
   unsigned bad = 0u;
@@ -403,6 +404,7 @@ constexpr int kRngChunk = 96, kRngSlot = 112;  // bytes; the slot holds an odd n
 constexpr int kRngWarpBytes = 1408 + 32 * kRngSlot;
 template <typename R, int MODE>
 __global__ void __launch_bounds__(128) rng_tile_kernel(const RngParams p) {
+  overlap_begin();
   __shared__ __align__(16) LogEntry table[kRngTable];
   __shared__ __align__(16) unsigned char area[4 * kRngWarpBytes];
   rng_load_table(table);
@@ -457,6 +459,7 @@ __global__ void __launch_bounds__(128) rng_tile_kernel(const RngParams p) {
 
 // S_*_seed_i_I: state k = QLA_seed_random(seed, a[k])
 static __global__ void __launch_bounds__(256) rng_seed_kernel(const RngParams p) {
+  overlap_begin();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < p.n;
        i += (long long)gridDim.x * blockDim.x) {
     const long long k = p.gang ? (long long)p.gang[i] : i;
@@ -469,6 +472,7 @@ static __global__ void __launch_bounds__(256) rng_seed_kernel(const RngParams p)
 
 // S_*_S and S_*_S_mask_I: 11 words per state, one thread per word
 static __global__ void __launch_bounds__(256) rng_copy_kernel(const RngParams p, int masked) {
+  overlap_begin();
   const long long total = p.n * 11;
   for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < total;
        g += (long long)gridDim.x * blockDim.x) {
@@ -511,9 +515,9 @@ inline void rng_launch_fill(const RngParams& p) {
   // (the tile kernel writes records in 8-B pieces)
   if (p.gang == nullptr && p.s.mode == OM_CONTIG &&
       (p.nreal == 1 || (reinterpret_cast<uintptr_t>(p.out) & 7u) == 0))
-    rng_tile_kernel<R, MODE><<<(unsigned)((p.n + 127) / 128), 128, 0, current_stream()>>>(p);
+    launch_kernel(rng_tile_kernel<R, MODE>, (unsigned)((p.n + 127) / 128), 128, 0, current_stream(), p);
   else
-    rng_fill_kernel<R, MODE><<<rng_grid(p.n, 128), 128, 0, current_stream()>>>(p);
+    launch_kernel(rng_fill_kernel<R, MODE>, rng_grid(p.n, 128), 128, 0, current_stream(), p);
 }
 
 // r (nreal reals per record of R) = uniform (gauss 0) or gaussian deviates
@@ -556,7 +560,7 @@ inline void api_rng_seed(const char* kid, void* r, int seed, Opnd a, const int* 
   }
   p.m = a;
   p.seed = seed;
-  rng_seed_kernel<<<rng_grid(n, 256), 256, 0, current_stream()>>>(p);
+  launch_kernel(rng_seed_kernel, rng_grid(n, 256), 256, 0, current_stream(), p);
   check_launch(kid);
 }
 
@@ -568,7 +572,7 @@ inline void api_rng_copy(const char* kid, void* r, Opnd a, Opnd mask, bool maske
     return;
   }
   p.m = mask;
-  rng_copy_kernel<<<rng_grid((long long)n * 11, 256), 256, 0, current_stream()>>>(p, masked ? 1 : 0);
+  launch_kernel(rng_copy_kernel, rng_grid((long long)n * 11, 256), 256, 0, current_stream(), p, masked ? 1 : 0);
   check_launch(kid);
 }
 

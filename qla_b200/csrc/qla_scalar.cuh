@@ -166,6 +166,7 @@ __device__ __forceinline__ R r_eqop(int eqop, R x, R t) {
 
 template <typename R, int OP>
 __global__ void __launch_bounds__(256) scalar_kernel(const ScParams p) {
+  overlap_begin();
   R sv = R(0);
   if constexpr (OP == SO_R_RTIMES || OP == SO_R_FILL || OP == SO_R_RT_PLUS || OP == SO_R_RT_MINUS)
     sv = p.sptr ? *static_cast<const R*>(p.sptr) : (R)p.sre;
@@ -329,7 +330,7 @@ inline void api_scalar(const char* kid, void* r, const void* scal, Opnd a, Opnd 
   const long long cap = (long long)device_sm_count() * 16;
   long long grid = ((long long)n + 255) / 256;
   if (grid > cap) grid = cap;
-  scalar_kernel<R, OP><<<(unsigned)(grid < 1 ? 1 : grid), 256, 0, current_stream()>>>(p);
+  launch_kernel(scalar_kernel<R, OP>, (unsigned)(grid < 1 ? 1 : grid), 256, 0, current_stream(), p);
   check_launch(kid);
 }
 
@@ -351,6 +352,7 @@ struct SredFinish {
 // integer fields below 2^53), each group added in double-double.
 template <typename RIN, typename RW, int KIND, typename OUT>
 __global__ void __launch_bounds__(256) sred_kernel(const EwParams p, const SiteParams rp) {
+  overlap_begin();
   constexpr int U = 8;
   DD acc[1] = {DD{0.0, 0.0}};
   auto term = [&](long long i) -> double {
@@ -415,7 +417,7 @@ inline void api_sred(const char* kid, void* r, Opnd a, Opnd b, const int* gang, 
   const long long cap = (long long)sms * 4;
   if (grid > cap) grid = cap;
   if (grid > rs->max_blocks) grid = rs->max_blocks;
-  sred_kernel<RIN, RW, KIND, OUT><<<(unsigned)(grid < 1 ? 1 : grid), 256, 0, st>>>(p, rp);
+  launch_kernel(sred_kernel<RIN, RW, KIND, OUT>, (unsigned)(grid < 1 ? 1 : grid), 256, 0, st, p, rp);
   if (!check_launch(kid)) return;
   if (!dev_out) {
     if (cudaMemcpyAsync(r, rs->result, rbytes, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
@@ -427,6 +429,7 @@ inline void api_sred(const char* kid, void* r, Opnd a, Opnd b, const int* gang, 
 // real precision conversion r = (ROUT) a
 template <typename RIN, typename ROUT>
 __global__ void __launch_bounds__(256) rconvert_kernel(const ScParams p) {
+  overlap_begin();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < p.n;
        i += (long long)gridDim.x * blockDim.x) {
     const long long k = p.gang ? (long long)p.gang[i] : i;
@@ -450,7 +453,7 @@ inline void api_rconvert(const char* kid, void* r, Opnd a, const int* gang, int 
   const long long cap = (long long)device_sm_count() * 16;
   long long grid = ((long long)n + 255) / 256;
   if (grid > cap) grid = cap;
-  rconvert_kernel<RIN, ROUT><<<(unsigned)(grid < 1 ? 1 : grid), 256, 0, current_stream()>>>(p);
+  launch_kernel(rconvert_kernel<RIN, ROUT>, (unsigned)(grid < 1 ? 1 : grid), 256, 0, current_stream(), p);
   check_launch(kid);
 }
 
