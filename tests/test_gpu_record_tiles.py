@@ -114,3 +114,51 @@ def test_padded_slot_products(qla, cuda, pc, nc):
         got = complex(*res.cpu().tolist())
         assert abs(got - np.vdot(z, z2)) <= 1e-12 * np.abs(z).sum() * np.abs(z2).max(), (nc, n)
     qla.check("padded slots")
+
+
+ADJOINT = ["M_veq_Ma", "M_vpeq_Ca_times_Ma", "M_vmeq_C_times_Ma", "M_veqm_c_times_Ma", "M_vpeq_r_times_Ma"]
+
+
+@pytest.mark.parametrize("pc", ["F3", "D3"])
+def test_adjoint_forms(qla, cuda, pc):
+    byname = {e["name"]: e for e in qla.manifest()}
+    rng = np.random.default_rng(61)
+    dt = np.float32 if pc == "F3" else np.float64
+    for n in SIZES + [2051]:
+        for short in ADJOINT:
+            e = byname[f"QLA_{pc}_{short}"]
+            ins, idx, gang = T.ewise_inputs(e, rng, dt, n, n)
+            want = T.ewise_oracle(e, ins, idx, gang, n)
+            for off in (0, 4, 8) if pc == "F3" else (0, 8):  # bytes past a 16-B boundary
+                assert T.bits_equal(_call(qla, cuda, e["name"], [], e, ins, n, off), want), (short, n, off)
+
+
+@pytest.mark.parametrize("pc,dt", [("F3", np.float32), ("D3", np.float64)])
+def test_small_field_tiles(qla, cuda, pc, dt):
+    """Volumes on both sides of the points where the tile size changes (the
+    64-site tiles, one usual tile per SM, one 64-site tile per SM of a
+    reduction) and with partial last tiles."""
+    sms = qla.lib().qlagpu_sm_count()
+    rng = np.random.default_rng(5)
+    top = 256 * sms + 65
+    a, b = T.haar_su3(rng, top, dt), T.gaussian_field(rng, top, 3, dt)
+    ad, bd = T.to_dev(a), T.to_dev(b)
+    h = T.positive_hermitian_inputs(rng, top, dt)
+    hd = T.to_dev(h)
+    ns_ = getattr(qla, pc)
+    want = np.zeros((top, 6), dt)
+    T.ora_lmult(want, a, b, top, 1, "eq")
+    for n in (1, 63, 64, 65, 64 * sms - 1, 64 * sms, 64 * sms + 33, 128 * sms, 256 * sms - 1, 256 * sms, top):
+        rd = T.to_dev(np.zeros((top, 6), dt))
+        ns_.V_veq_M_times_V(rd, ad, bd, n)
+        got = T.to_host(rd)
+        assert T.bits_equal(got[:n], want[:n]) and not got[n:].any(), n
+        nrm = getattr(qla, "DF3" if pc == "F3" else "D3").r_veq_norm2_V(None, bd, n)
+        exact = T.ora_norm2(b, n, 3, exact=True)
+        assert abs(nrm - exact) <= 1e-12 * exact, n
+        xd = T.to_dev(np.zeros((top, 18), dt))
+        ns_.M_veq_inverse_M(xd, hd, n)
+        inv = T.to_host(xd)
+        if n <= 64 * sms:
+            assert T.bits_equal(inv[:n], T.ora_mfunc(np.ascontiguousarray(h[:n]), n, "inverse")), n
+        assert not inv[n:].any(), n
