@@ -461,6 +461,12 @@ template <class OP>
 struct ComputeBound {
   static constexpr bool value = false;
 };
+// Operators whose arithmetic hides behind the movement of their records even
+// with half the usual warps (specialised beside them).
+template <class OP>
+struct StreamsRecords {
+  static constexpr bool value = false;
+};
 // Blocks of 128 threads an SM must hold, by the 32-bit registers that one
 // site's records fill: 5 (102 registers), 3 (168) or 1 (255).  (Left to itself
 // the compiler spills the 8-colour matrix products: 211 us against 55.)

@@ -115,6 +115,113 @@ struct SiteLauncher {
                                 OP::N2 * (int)sizeof(Cx<R>)};
   static constexpr int OB = OP::NOUT * (int)sizeof(Cx<R>);
 
+  // Everything about a launch that does not depend on the arrays or n.
+  struct Shape {
+    // what it was made for
+    const char* kernel_id = nullptr;
+    int device = -1, modes = -1;
+    unsigned version = 0;
+    // the shape
+    int threads, stages, blocks;  // blocks: resident per SM
+    size_t smem;
+    unsigned off_in[3], off_out_in, tx_bytes, stage_bytes;
+  };
+
+  // Warp-cooperative kernel: four warps a block, fewer where their slices would
+  // leave less than four blocks an SM.  (Kept per host thread and device, like
+  // tile_shape's: with the locked tables behind the tuning, the occupancy and the
+  // shared-memory limit on every call, 24 short calls took 100 us, 96 so.)
+  static const Shape& coop_shape() {
+    static thread_local Shape sh;
+    const int dev = current_device();
+    if (sh.device == dev) return sh;
+    constexpr unsigned wb = CoopLayout<OP>::warp_bytes;
+    int nw = 4;
+    while (nw > 1 && nw * wb > 48u * 1024u) nw /= 2;
+    sh.threads = 32 * nw;
+    sh.smem = (size_t)nw * wb;
+    const void* fn = reinterpret_cast<const void*>(&site_coop_kernel<OP>);
+    launch_smem_limit(fn, sh.smem);
+    sh.blocks = launch_blocks_per_sm(fn, sh.threads, sh.smem);
+    sh.device = dev;
+    return sh;
+  }
+
+  // Bulk-copy kernel, for p's operand modes and whether the destination is
+  // read: the autotuner's shape (or the default; SMALL: two stages of 64 sites)
+  // and the stage layout.  Remade when the tuning table changes (tune_version).
+  template <bool SMALL>
+  static const Shape& tile_shape(const SiteParams& p, const char* kernel_id) {
+    static thread_local Shape sh;
+    const int dev = current_device();
+    int modes = OP::NOUT > 0 && p.out_read ? 1 : 0;
+    for (int j = 0; j < OP::NIN; j++) modes = modes * 4 + (p.in[j].mode & 3);
+    const unsigned version = tune_version();
+    if (sh.device == dev && sh.modes == modes && sh.version == version && sh.kernel_id == kernel_id) return sh;
+    unsigned bps = 0;
+    for (int j = 0; j < OP::NIN; j++)
+      bps += p.in[j].mode == OM_CONTIG ? RB[j] : (p.in[j].mode == OM_PTR ? 8u : 4u);
+    if (OP::NOUT > 0 && p.out_read) bps += OB;
+    LaunchShape ls = default_shape(bps, OB);
+    int tt, ts;
+    char key[96];
+    {
+      int q = 0;
+      for (const char* c = kernel_id; *c && q < 80; c++) key[q++] = *c;
+      key[q++] = ':';
+      for (int j = 0; j < OP::NIN; j++) key[q++] = "-cpi"[p.in[j].mode & 3];
+      if (OP::NOUT > 0 && p.out_read) key[q++] = 'r';
+      key[q] = 0;
+    }
+    if (SMALL) {
+      ls.threads = 64;
+      ls.stages = 2;
+    } else if (tuned_shape(key, &tt, &ts)) {
+      ls.threads = tt;
+      ls.stages = ts;
+    }
+    // stay within the per-block shared-memory limit (227 KB less the static
+    // reduction scratch): shed stages, then halve the tile down to one warp,
+    // then (very large records, e.g. nc = 8 matrices) run unpipelined
+    while (tma_smem_bytes(ls.threads, ls.stages, stage_bytes_for(ls.threads, bps), OB) > 225u * 1024u) {
+      if (ls.stages > 2)
+        ls.stages--;
+      else if (ls.threads > 32)
+        ls.threads /= 2;
+      else if (ls.stages > 1)
+        ls.stages = 1;
+      else
+        break;
+    }
+    const int T = ls.threads;
+    unsigned off = 0;
+    sh.tx_bytes = 0;
+    for (int j = 0; j < 3; j++) sh.off_in[j] = 0;
+    for (int j = 0; j < OP::NIN; j++) {
+      sh.off_in[j] = off;
+      const unsigned b = (unsigned)T * (p.in[j].mode == OM_CONTIG ? RB[j] : (p.in[j].mode == OM_PTR ? 8u : 4u));
+      off += (b + 15u) & ~15u;
+      sh.tx_bytes += b;
+    }
+    sh.off_out_in = off;
+    if (OP::NOUT > 0 && p.out_read) {
+      off += (unsigned)T * OB;
+      sh.tx_bytes += (unsigned)T * OB;
+    }
+    sh.stage_bytes = (off + 127u) & ~127u;
+    sh.threads = T;
+    sh.stages = ls.stages;
+    sh.smem = tma_smem_bytes(T, sh.stages, sh.stage_bytes, OB);
+    const void* fn = reinterpret_cast<const void*>(&site_tma_kernel<OP>);
+    launch_smem_limit(fn, sh.smem);
+    sh.blocks = launch_blocks_per_sm(fn, T + 32, sh.smem);
+    sh.device = dev;
+    sh.modes = modes;
+    sh.version = version;
+    sh.kernel_id = kernel_id;
+    return sh;
+  }
+
   // kernel_id names the OP for the autotuner table
   static void run(SiteParams p, const char* kernel_id, void* host_result = nullptr, size_t result_bytes = 0) {
     constexpr bool reduce = OP::NACC > 0;
@@ -160,86 +267,46 @@ struct SiteLauncher {
       if (host_result) p.result = rs->result;
     }
 
+    // Small fields run 64-site tiles: more SMs get a tile and the last round is
+    // emptier by less.  Operators that only stream records: below three rounds
+    // of the usual tiles (24 calls of a Wilson hop in a graph, usual / 64-site
+    // tiles, us: 16^4 sites 90 / 87, 16^3 x 32 127 / 107, 24^4 242 / 232, but
+    // 24^3 x 48 470 / 469 and 32^4 739 / 754).  Arithmetic suffers from a producer
+    // warp for every two consumers (F3 sqrtPH at 65,536 sites 5.2 / 5.9, at 4,096
+    // 3.9 / 3.2): while there are fewer usual tiles than SMs.  Reductions fold one
+    // partial per block (F3 norm2_D at 65,536 sites 5.4 / 8.9, at 4,096 4.5 / 4.1):
+    // while the 64-site tiles do not outnumber the SMs.
+    const Shape* ps = direct ? &coop_shape() : &tile_shape<false>(p, kernel_id);
+    if (!direct && ps->threads > 64) {
+      const long long usual = (long long)ps->threads * sms;
+      const long long below = reduce ? 64LL * sms : StreamsRecords<OP>::value ? 3 * usual * ps->blocks : usual;
+      if (p.n < below) ps = &tile_shape<true>(p, kernel_id);
+    }
+    const Shape& sh = *ps;
+    long long grid;
+    cudaError_t rc;
     if (direct) {
-      // four warps a block, fewer where their slices would leave less than
-      // four blocks an SM
-      constexpr unsigned wb = CoopLayout<OP>::warp_bytes;
-      int nw = 4;
-      while (nw > 1 && nw * wb > 48u * 1024u) nw /= 2;
-      const size_t smem = (size_t)nw * wb;
-      const void* fn = reinterpret_cast<const void*>(&site_coop_kernel<OP>);
-      launch_smem_limit(fn, smem);
-      long long grid = (p.n + 32 * nw - 1) / (32 * nw);
-      const long long cap = (long long)launch_blocks_per_sm(fn, 32 * nw, smem) * sms;
-      if (grid > cap) grid = cap;
+      grid = (p.n + sh.threads - 1) / sh.threads;
+      if (grid > (long long)sh.blocks * sms) grid = (long long)sh.blocks * sms;
       if (reduce && grid > rs->max_blocks) grid = rs->max_blocks;
-      if (launch_kernel(&site_coop_kernel<OP>, (unsigned)grid, 32u * nw, smem, st, p) != cudaSuccess) {
-        check_launch(kernel_id);
-        return;
-      }
+      rc = launch_kernel(&site_coop_kernel<OP>, (unsigned)grid, (unsigned)sh.threads, sh.smem, st, p);
     } else {
-      unsigned bps = 0;
-      for (int j = 0; j < OP::NIN; j++)
-        bps += p.in[j].mode == OM_CONTIG ? RB[j] : (p.in[j].mode == OM_PTR ? 8u : 4u);
-      if (OP::NOUT > 0 && p.out_read) bps += OB;
-      LaunchShape sh = default_shape(bps, OB);
-      int tt, ts;
-      char key[96];
-      {
-        int q = 0;
-        for (const char* c = kernel_id; *c && q < 80; c++) key[q++] = *c;
-        key[q++] = ':';
-        for (int j = 0; j < OP::NIN; j++) key[q++] = "-cpi"[p.in[j].mode & 3];
-        if (OP::NOUT > 0 && p.out_read) key[q++] = 'r';
-        key[q] = 0;
-      }
-      if (tuned_shape(key, &tt, &ts)) {
-        sh.threads = tt;
-        sh.stages = ts;
-      }
-      // stay within the per-block shared-memory limit (227 KB less the static
-      // reduction scratch): shed stages, then halve the tile down to one warp,
-      // then (very large records, e.g. nc = 8 matrices) run unpipelined
-      while (tma_smem_bytes(sh.threads, sh.stages, stage_bytes_for(sh.threads, bps), OB) > 225u * 1024u) {
-        if (sh.stages > 2)
-          sh.stages--;
-        else if (sh.threads > 32)
-          sh.threads /= 2;
-        else if (sh.stages > 1)
-          sh.stages = 1;
-        else
-          break;
-      }
-      const int T = sh.threads;
-      unsigned off = 0;
-      p.tx_bytes = 0;
-      for (int j = 0; j < OP::NIN; j++) {
-        p.off_in[j] = off;
-        unsigned b = (unsigned)T * (p.in[j].mode == OM_CONTIG ? RB[j] : (p.in[j].mode == OM_PTR ? 8u : 4u));
-        off += (b + 15u) & ~15u;
-        p.tx_bytes += b;
-      }
-      p.off_out_in = off;
-      if (OP::NOUT > 0 && p.out_read) {
-        off += (unsigned)T * OB;
-        p.tx_bytes += (unsigned)T * OB;
-      }
-      p.stage_bytes = (off + 127u) & ~127u;
-      p.ntiles = p.n / T;
+      for (int j = 0; j < 3; j++) p.off_in[j] = sh.off_in[j];
+      p.off_out_in = sh.off_out_in;
+      p.tx_bytes = sh.tx_bytes;
+      p.stage_bytes = sh.stage_bytes;
       p.stages = sh.stages;
-      const size_t smem = tma_smem_bytes(T, p.stages, p.stage_bytes, OB);
-      const void* fn = reinterpret_cast<const void*>(&site_tma_kernel<OP>);
-      launch_smem_limit(fn, smem);
-      const int nb = launch_blocks_per_sm(fn, T + 32, smem);
-      long long grid = (long long)nb * sms;
+      p.ntiles = p.n / sh.threads;
+      grid = (long long)sh.blocks * sms;
       if (grid > p.ntiles) grid = p.ntiles;
       if (grid < 1) grid = 1;
       if (reduce && grid > rs->max_blocks) grid = rs->max_blocks;
-      // T consumer threads + one producer warp
-      if (launch_kernel(&site_tma_kernel<OP>, (unsigned)grid, (unsigned)T + 32u, smem, st, p) != cudaSuccess) {
-        check_launch(kernel_id);
-        return;
-      }
+      // threads consumers (one site each per tile) + one producer warp
+      rc = launch_kernel(&site_tma_kernel<OP>, (unsigned)grid, (unsigned)sh.threads + 32u, sh.smem, st, p);
+    }
+    if (rc != cudaSuccess) {
+      check_launch(kernel_id);
+      return;
     }
     if (!check_launch(kernel_id)) return;
     if (reduce && host_result) {

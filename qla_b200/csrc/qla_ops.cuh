@@ -424,4 +424,38 @@ struct ReDotOp {
   __device__ static void finish(const SiteParams& p, const double* tot) { write_real<OUT>(p, tot[0]); }
 };
 
+// operators that only stream records (tile size of small fields)
+template <typename R, int NC, int NCOL, bool ADJA, bool ADJB>
+struct StreamsRecords<LMultOp<R, NC, NCOL, ADJA, ADJB>> {
+  static constexpr bool value = true;
+};
+template <typename R, int NC>
+struct StreamsRecords<SpprojOp<R, NC>> {
+  static constexpr bool value = true;
+};
+template <typename R, int NC>
+struct StreamsRecords<SpreconOp<R, NC>> {
+  static constexpr bool value = true;
+};
+template <typename R, int NC, bool ADJA, int DEST>
+struct StreamsRecords<SpprojMultOp<R, NC, ADJA, DEST>> {
+  static constexpr bool value = true;
+};
+template <typename R, int NC, bool ADJA>
+struct StreamsRecords<SpreconMultOp<R, NC, ADJA>> {
+  static constexpr bool value = true;
+};
+template <typename R, int NC>
+struct StreamsRecords<SpprojDOp<R, NC>> {
+  static constexpr bool value = true;
+};
+template <typename R, int N>
+struct StreamsRecords<RTimesOp<R, N>> {
+  static constexpr bool value = true;
+};
+template <typename R, int N>
+struct StreamsRecords<CopyOp<R, N>> {
+  static constexpr bool value = true;
+};
+
 }  // namespace qlab

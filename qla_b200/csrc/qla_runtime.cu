@@ -58,16 +58,20 @@ int current_device() {
   return d;
 }
 
+// (the first kMaxFast devices without a lock: every call asks)
+constexpr int kMaxFast = 64;
+
 int device_sm_count() {
-  static std::mutex mu;
-  static std::map<int, int> cache;
+  static std::atomic<int> cache[kMaxFast];
   const int d = current_device();
-  std::lock_guard<std::mutex> g(mu);
-  auto it = cache.find(d);
-  if (it != cache.end()) return it->second;
+  const bool fast = d >= 0 && d < kMaxFast;
+  if (fast) {
+    const int n = cache[d].load(std::memory_order_relaxed);
+    if (n > 0) return n;
+  }
   int sms = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d) != cudaSuccess || sms <= 0) sms = 1;
-  cache[d] = sms;
+  if (fast) cache[d].store(sms, std::memory_order_relaxed);
   return sms;
 }
 
@@ -93,7 +97,12 @@ std::map<std::pair<int, cudaStream_t>, ReduceScratch> g_scratch;
 }  // namespace
 
 unsigned* device_error_word() {
+  static std::atomic<unsigned*> cache[kMaxFast];
   const int d = current_device();
+  const bool fast = d >= 0 && d < kMaxFast;
+  if (fast) {
+    if (unsigned* p = cache[d].load(std::memory_order_acquire)) return p;
+  }
   std::lock_guard<std::mutex> g(g_mu);
   DevState& s = g_dev[d];
   if (!s.err) {
@@ -106,6 +115,7 @@ unsigned* device_error_word() {
     cudaMemset(p, 0, sizeof(unsigned));
     s.err = p;
   }
+  if (fast) cache[d].store(s.err, std::memory_order_release);
   return s.err;
 }
 
@@ -141,7 +151,10 @@ namespace {
 std::mutex g_tune_mu;
 std::map<std::string, std::pair<int, int>> g_tune;
 std::atomic<int> g_tune_count{0};
+std::atomic<unsigned> g_tune_version{1};
 }  // namespace
+
+unsigned tune_version() { return g_tune_version.load(std::memory_order_acquire); }
 
 // The shipped table (tune_b200.txt beside the package, written by
 // `python -m qla_b200.tune` on a B200) or the file named by $QLA_B200_TUNE is
@@ -289,6 +302,7 @@ QLAB_EXPORT int qlagpu_tune_set(const char* kernel_id, int threads, int stages) 
   std::lock_guard<std::mutex> g(g_tune_mu);
   g_tune[kernel_id] = std::make_pair(threads, stages);
   g_tune_count.store((int)g_tune.size());
+  g_tune_version.fetch_add(1, std::memory_order_release);
   return QLAGPU_OK;
 }
 
@@ -297,6 +311,7 @@ QLAB_EXPORT void qlagpu_tune_clear(void) {
   std::lock_guard<std::mutex> g(g_tune_mu);
   g_tune.clear();
   g_tune_count.store(0);
+  g_tune_version.fetch_add(1, std::memory_order_release);
 }
 
 QLAB_EXPORT int qlagpu_sm_count(void) { return device_sm_count(); }

@@ -38,6 +38,8 @@ ReduceScratch* reduce_scratch(cudaStream_t st, int max_blocks);
 // launch-shape override from the autotuner (qlagpu_tune_set): returns false
 // when no override exists for this kernel id.
 bool tuned_shape(const char* kernel_id, int* threads, int* stages);
+// changes with every change of the table
+unsigned tune_version();
 
 // the current device's error word (device memory, zero-initialised)
 unsigned* device_error_word();
