@@ -173,12 +173,24 @@ struct SiteLauncher {
       if (OP::NOUT > 0 && p.out_read) key[q++] = 'r';
       key[q] = 0;
     }
+    const void* fn = reinterpret_cast<const void*>(&site_tma_kernel<OP>);
     if (SMALL) {
       ls.threads = 64;
       ls.stages = 2;
     } else if (tuned_shape(key, &tt, &ts)) {
       ls.threads = tt;
       ls.stages = ts;
+    } else {
+      // Where registers, not shared memory, limit the blocks on an SM, a block of
+      // nine warps may leave room for much less than another one: half the
+      // tile if at least a quarter more consumers fit (F3 reunit at 104
+      // registers, 24^3 x 48: 8 consumer warps 49 us, 12 so 41; sqrt 110 / 98).
+      auto consumers = [&](int t) {
+        const size_t m = tma_smem_bytes(t, ls.stages, stage_bytes_for(t, bps), OB);
+        launch_smem_limit(fn, m);
+        return t * launch_blocks_per_sm(fn, t + 32, m);
+      };
+      while (ls.threads > 64 && 4 * consumers(ls.threads / 2) >= 5 * consumers(ls.threads)) ls.threads /= 2;
     }
     // stay within the per-block shared-memory limit (227 KB less the static
     // reduction scratch): shed stages, then halve the tile down to one warp,
@@ -212,7 +224,6 @@ struct SiteLauncher {
     sh.threads = T;
     sh.stages = ls.stages;
     sh.smem = tma_smem_bytes(T, sh.stages, sh.stage_bytes, OB);
-    const void* fn = reinterpret_cast<const void*>(&site_tma_kernel<OP>);
     launch_smem_limit(fn, sh.smem);
     sh.blocks = launch_blocks_per_sm(fn, T + 32, sh.smem);
     sh.device = dev;
