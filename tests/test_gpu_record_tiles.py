@@ -162,3 +162,23 @@ def test_small_field_tiles(qla, cuda, pc, dt):
         if n <= 64 * sms:
             assert T.bits_equal(inv[:n], T.ora_mfunc(np.ascontiguousarray(h[:n]), n, "inverse")), n
         assert not inv[n:].any(), n
+
+
+@pytest.mark.parametrize("pc,dt", [("F3", np.float32), ("D3", np.float64)])
+@pytest.mark.parametrize("n", [63, 65, 18943, 18945, 19071, 37889])
+def test_register_limited_operators_take_smaller_tiles(qla, pc, dt, n):
+    """Matrix functions whose registers limit the blocks on an SM, contiguous and
+    through a pointer array, around one and two 128-site tiles per SM."""
+    rng = np.random.default_rng(91 + n)
+    a = T.positive_hermitian_inputs(rng, n, np.float64).astype(dt)
+    idx = rng.permutation(n).astype(np.int32)
+    ns_ = getattr(qla, pc)
+    a_d = T.to_dev(a)
+    ptrs = T.ptr_array(a_d, idx, 9 * 2 * np.dtype(dt).itemsize)
+    for fname in ("sqrt", "invsqrt"):
+        r = T.to_dev(np.zeros_like(a))
+        getattr(ns_, f"M_veq_{fname}_M")(r, a_d, n)
+        want = T.ora_mfunc(a, n, fname)
+        assert T.bits_equal(T.to_host(r), want), fname
+        getattr(ns_, f"M_veq_{fname}_pM")(r, ptrs, n)
+        assert T.bits_equal(T.to_host(r), want[idx]), fname + " pM"
