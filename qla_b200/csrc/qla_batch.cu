@@ -426,8 +426,12 @@ __global__ void __launch_bounds__(128, 4) batch_program_kernel(const BatchParams
           cp_async_wait_all();
           bulk_wait_read<0>();  // the previous tile's results have left their slots
           if (!mbar_wait_bounded(&bar[place(cnt)], parity(cnt), p.err)) alive = false;
-          alive = __all_sync(0xffffffffu, alive);  // this tile's records and the next tile's indices have landed
+          alive = __all_sync(0xffffffffu, alive);
           if (!alive) break;
+          // this tile's records and the next tile's indices have landed; a lane's
+          // cp.async copies and zeroed records show to the others only behind this
+          // barrier (a vote does not order memory)
+          __syncwarp();
           const unsigned q1 = q == 2u ? 0u : q + 1u, q2 = q1 == 2u ? 0u : q1 + 1u;
           unsigned char* stage = stages + place(cnt) * p.stage_bytes;
           if (p.stages == 2 && t + nw < tend)
