@@ -463,7 +463,10 @@ __global__ void __launch_bounds__(128, 4) batch_program_kernel(const BatchParams
                 run_out(S.base + (size_t)t * 32u * rb, stage + S.out,
                         (unsigned)nv * rb, lane);
             }
-            __syncwarp();  // the result slots are free
+            // the result slots are free: this lane's reads of them come before
+            // the bulk copies that fill them next
+            fence_proxy_async_smem();
+            __syncwarp();
           }
           if (p.stages == 1 && t + nw < tend) {
             bulk_wait_read<0>();
