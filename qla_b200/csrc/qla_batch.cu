@@ -412,9 +412,14 @@ __global__ void __launch_bounds__(128, 4) batch_program_kernel(const BatchParams
           if (S.used && !S.idx) L.in = at;
           if (S.role != BR_IN) L.out = at;
         }
-        // fill the pipeline: indices of two tiles, records of the first
+        // fill the pipeline: indices of two tiles, records of the first.  The
+        // last results of the field or run before may still be leaving the
+        // stage (in a one-stage plan it is the one filled now, and the tile loop
+        // waits for them only when it has another tile to fetch): every lane
+        // waits until its bulk stores have read their slots, then all go on
         unsigned q = 0;  // ring place of tile t's indices
         fetch_indices(F, area, t, 0, sites(t), lane);
+        bulk_wait_read<0>();
         cp_async_wait_all();
         __syncwarp();
         // stage and barrier of the c-th tile this warp fetches, and its parity
