@@ -727,7 +727,7 @@ __global__ void __launch_bounds__(1024, 2) gsum_kernel(const EwParams p, DD* par
 constexpr int GS_FOLD = 128;
 
 template <typename OUT>
-__global__ void __launch_bounds__(GS_FOLD) gsum_fold_kernel(const DD* __restrict__ partials, int nblk, int nr,
+__global__ void __launch_bounds__(GS_FOLD) gsum_fold_kernel(const DD* partials, int nblk, int nr,
                                                             OUT* result) {
   overlap_begin();
   __shared__ DD red[GS_FOLD];
