@@ -100,6 +100,25 @@ __device__ __forceinline__ T ld_in(const T* p) {
   return *p;
 }
 
+// A load of an input that is issued where it stands among the other loads, waits
+// and copies (volatile, so never above overlap_begin), and that no store or local
+// array before it can alias.
+__device__ __forceinline__ float2 ld_here(const float2* p) {
+  float2 v;
+  asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double2 ld_here(const double2* p) {
+  double2 v;
+  asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float4 ld_here(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+
 // ---------------------------------------------------------------------------
 // record movement.  A record of N complex numbers of type R lives at an
 // address aligned to sizeof(Cx<R>) (8 B for float, 16 B for double).

@@ -223,6 +223,14 @@ __global__ void __launch_bounds__(256) ew_flat_kernel(const EwParams p, long lon
       return s;
     }
   };
+  // With a complex scalar field the loads are issued together (ld_here): left to the
+  // compiler, which takes 32 registers where __ldg took 40, they come late.  Without
+  // one it does better itself.  (us: QLA_F3_D_vpeq_C_times_D on 666,666 sites __ldg
+  // 27, plain loads 37, so 25, on 2.8 M 126 / 161 / 124; QLA_D3_D_veq_conj_D on
+  // 333,333 plain loads 19, so 21.)
+  constexpr bool HERE = SCAL == SC_FIELD && !SREAL;
+  auto load2 = [](const double2* q) { return HERE ? ld_here(q) : ld_in(q); };
+  auto load4 = [](const float4* q) { return HERE ? ld_here(q) : ld_in(q); };
   const long long nvec = nelem / CPT;
   for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < nvec;
        v += (long long)gridDim.x * blockDim.x) {
@@ -232,11 +240,11 @@ __global__ void __launch_bounds__(256) ew_flat_kernel(const EwParams p, long lon
     for (int h = 0; h < 2; h++) {
       const long long q = g0 + h * CPV;
       if constexpr (sizeof(R) == 4) {
-        const float4 u = ld_in(reinterpret_cast<const float4*>(B + q));
+        const float4 u = load4(reinterpret_cast<const float4*>(B + q));
         b[2 * h] = Cx<R>{u.x, u.y};
         b[2 * h + 1] = Cx<R>{u.z, u.w};
         if constexpr (TWO) {
-          const float4 w = ld_in(reinterpret_cast<const float4*>(C + q));
+          const float4 w = load4(reinterpret_cast<const float4*>(C + q));
           c[2 * h] = Cx<R>{w.x, w.y};
           c[2 * h + 1] = Cx<R>{w.z, w.w};
         }
@@ -246,10 +254,10 @@ __global__ void __launch_bounds__(256) ew_flat_kernel(const EwParams p, long lon
           x[2 * h + 1] = Cx<R>{o.z, o.w};
         }
       } else {
-        const double2 u = ld_in(reinterpret_cast<const double2*>(B + q));
+        const double2 u = load2(reinterpret_cast<const double2*>(B + q));
         b[h] = Cx<R>{u.x, u.y};
         if constexpr (TWO) {
-          const double2 w = ld_in(reinterpret_cast<const double2*>(C + q));
+          const double2 w = load2(reinterpret_cast<const double2*>(C + q));
           c[h] = Cx<R>{w.x, w.y};
         }
         if (load) {
