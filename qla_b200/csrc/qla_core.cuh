@@ -196,6 +196,21 @@ __device__ __forceinline__ void load_rec_global(Cx<R> (&x)[N], const void* p) {
   }
 }
 
+// the same with loads that are issued where they stand (ld_here)
+template <typename R, int N>
+__device__ __forceinline__ void load_rec_here(Cx<R> (&x)[N], const void* p) {
+#pragma unroll
+  for (int e = 0; e < N; e++) {
+    if constexpr (sizeof(R) == 4) {
+      const float2 v = ld_here(static_cast<const float2*>(p) + e);
+      x[e] = Cx<R>{v.x, v.y};
+    } else {
+      const double2 v = ld_here(static_cast<const double2*>(p) + e);
+      x[e] = Cx<R>{v.x, v.y};
+    }
+  }
+}
+
 // plain global load (used where the record may alias the output, i.e. the
 // destination of a peq/meq update)
 template <typename R, int N>

@@ -77,7 +77,10 @@ __device__ __forceinline__ void fetch_gathered(Cx<typename OP::R> (&x)[ArrN<N>::
     src = static_cast<const char*>(o.base) + (long long)o.idx[k] * RB;
   else
     src = static_cast<const char*>(o.base) + k * RB;
-  load_rec_global<R, ArrN<N>::value>(x, src);
+  if constexpr (OP::NIN > 1)
+    load_rec_here<R, ArrN<N>::value>(x, src);
+  else
+    load_rec_global<R, ArrN<N>::value>(x, src);
 }
 
 // Direct path: all operands read straight from global memory for site k.
@@ -461,6 +464,13 @@ template <class OP>
 struct ComputeBound {
   static constexpr bool value = false;
 };
+// Operators that run one site per thread on global memory (specialised beside
+// them): `contiguous` for aligned arrays too, `scattered` for gang-index calls
+// and operands off a 16-B boundary.
+template <class OP>
+struct SitePerThread {
+  static constexpr bool contiguous = false, scattered = false;
+};
 // Operators whose arithmetic hides behind the movement of their records even
 // with half the usual warps (specialised beside them).
 template <class OP>
@@ -543,7 +553,13 @@ __global__ void __launch_bounds__(128, coop_min_blocks<OP>()) site_coop_kernel(c
   if constexpr (OP::NACC > 0) reduce_finish<OP>(p, dacc);
 }
 
-// One site per thread, for the allocation-free entry point's unaligned calls.
+// Kernel 3: one site per thread, records read and written where they lie, up to
+// 255 registers a thread.  For operators whose arithmetic on one site outweighs
+// its bytes and needs more registers, or more local memory, than the warps that
+// share shared-memory slots can have (SitePerThread), and for the allocation-free
+// entry point's unaligned calls.  Operators of two inputs load with ld_here: into
+// local arrays, plain loads of the second record wait for the first one's stores
+// (QLA_DN_M_xeq_M_inverse_M, nc = 8, 23,438 sites: 159 us with __ldg, 237 plain).
 template <class OP>
 __global__ void __launch_bounds__(256) site_direct_kernel(const SiteParams p) {
   overlap_begin();

@@ -233,6 +233,28 @@ struct SiteLauncher {
     return sh;
   }
 
+  // the launch has been made: its status, and a reduction's result on the host
+  static void finish_call(const ReduceScratch* rs, const char* kernel_id, void* host_result, size_t result_bytes) {
+    if (!check_launch(kernel_id) || OP::NACC == 0 || !host_result) return;
+    cudaStream_t st = current_stream();
+    if (cudaMemcpyAsync(host_result, rs->result, result_bytes, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess)
+      check_launch(kernel_id);
+  }
+
+  // One site per thread, in blocks of 256; of fewer threads (32 at least) while
+  // blocks of twice as many would leave SMs without one (QLA_DN_M_veq_invsqrt_M,
+  // nc = 8, 3,000 sites: blocks of 256 1,012 us, so 269).
+  static void run_per_site(const SiteParams& p, const char* kernel_id, int sms, const ReduceScratch* rs,
+                           void* host_result, size_t result_bytes) {
+    int threads = 256;
+    while (threads > 32 && p.n <= (long long)threads / 2 * sms) threads /= 2;
+    long long grid = (p.n + threads - 1) / threads;
+    if (grid > 8LL * sms) grid = 8LL * sms;
+    launch_kernel(&site_direct_kernel<OP>, (unsigned)grid, (unsigned)threads, 0, current_stream(), p);
+    finish_call(rs, kernel_id, host_result, result_bytes);
+  }
+
   // kernel_id names the OP for the autotuner table
   static void run(SiteParams p, const char* kernel_id, void* host_result = nullptr, size_t result_bytes = 0) {
     constexpr bool reduce = OP::NACC > 0;
@@ -249,13 +271,15 @@ struct SiteLauncher {
     }
     p.err = device_error_word();
     // ---- path selection
-    bool direct = (p.gang != nullptr);  // the warp-cooperative kernel
+    bool scattered = (p.gang != nullptr);
     for (int j = 0; j < OP::NIN; j++) {
       const Opnd& o = p.in[j];
       const void* q = o.mode == OM_PTR ? (const void*)o.ptrs : (o.mode == OM_IDX ? (const void*)o.idx : o.base);
-      if (!aligned16(q)) direct = true;
+      if (!aligned16(q)) scattered = true;
     }
-    if (OP::NOUT > 0 && !aligned16(p.out)) direct = true;
+    if (OP::NOUT > 0 && !aligned16(p.out)) scattered = true;
+    const bool per_site = scattered ? SitePerThread<OP>::scattered : SitePerThread<OP>::contiguous;
+    bool direct = scattered;  // the warp-cooperative kernel
     // Records of a multiple of 128 B (4 and 8 colours' matrices and Dirac
     // fermions) lie flat in a bulk-copied tile with all eight lanes of a phase
     // on the same banks; the warp-cooperative kernel pads its slots.  Measured
@@ -276,6 +300,11 @@ struct SiteLauncher {
       p.partials = rs->partials;
       p.counter = rs->counter;
       if (host_result) p.result = rs->result;
+    }
+
+    if (per_site) {
+      run_per_site(p, kernel_id, sms, rs, host_result, result_bytes);
+      return;
     }
 
     // Small fields run 64-site tiles: more SMs get a tile and the last round is
@@ -319,12 +348,7 @@ struct SiteLauncher {
       check_launch(kernel_id);
       return;
     }
-    if (!check_launch(kernel_id)) return;
-    if (reduce && host_result) {
-      if (cudaMemcpyAsync(host_result, rs->result, result_bytes, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-          cudaStreamSynchronize(st) != cudaSuccess)
-        check_launch(kernel_id);
-    }
+    finish_call(rs, kernel_id, host_result, result_bytes);
   }
 };
 

@@ -304,9 +304,43 @@ struct GenDetOp {
   __device__ static void finish(const SiteParams&, const double*) {}
 };
 
-// (arithmetic on NC x NC matrices, at nc = 8 in local memory; bulk-copy kernel
-// / warp-cooperative, us: nc = 4 on 320,000 sites 130 / 123, nc = 8 on 41,472
-// sites 570 / 467)
+// Matrix functions of four and more colours: their work matrices take 255
+// registers or local memory, and warps that also hold the records of 32 sites in
+// shared memory are too few (nc = 8) or have too few registers (nc = 4, float).
+// Measured, us, bulk-copy tiles / warp-cooperative / one site per thread, on 48 MB
+// of matrices (FN nc = 4 375,000 sites, DN nc = 4 187,500, FN nc = 8 93,750, DN nc =
+// 8 46,875):
+//   sqrt   FN4 228 / 304 / 214   DN4 613 / 464 / 240   FN8 1546 / 1959 / 829
+//   inverse    148 / 107 / 100       169 / 116 / 89         332 / 599 / 298
+//   invsqrt    547 / 390 / 273       743 / 560 / 290       2358 / 3132 / 1244
+//   a^-1 b     161 / 113 / 131       193 / 141 / 103        908 / 565 / 252
+//   exp        154 / 141 / 167       284 / 228 / 144       1333 / 1057 / 627
+//   log       1131 / 864 / 1270     2783 / 2009 / 859      7970 / 9046 / 4782
+//   eigenvals  339 / 370 / 282       427 / 447 / 338       2470 / 1383 / 948
+//   det         49 / 26 / 39          53 / 27 / 32          169 / 98 / 84
+// Gang forms (half the sites), warp-cooperative / one site per thread: FN4 sqrt 153
+// / 97, log 431 / 650, exp 69 / 87, det 16 / 21; DN4 sqrt 235 / 125, DN8 sqrt 2182 /
+// 1057, a^-1 b 477 / 163; FN3 exp 56 / 48, log 280 / 240; F3 log 170 / 131.  det and,
+// in FN4, exp, log and contiguous a^-1 b stay in the warps' slots.
+template <typename R, int NC>
+struct SitePerThread<GenSqrtOp<R, NC>> {
+  static constexpr bool contiguous = NC >= 4, scattered = NC >= 4;
+};
+template <typename R, int NC>
+struct SitePerThread<GenInverseOp<R, NC>> {
+  static constexpr bool contiguous = NC >= 4, scattered = NC >= 4;
+};
+template <typename R, int NC>
+struct SitePerThread<GenExpOp<R, NC>> {
+  static constexpr bool contiguous = NC >= 4 && !(NC == 4 && sizeof(R) == 4),
+                        scattered = contiguous || (NC == 3 && sizeof(R) == 4);
+};
+template <typename R, int NC>
+struct SitePerThread<GenDetOp<R, NC>> {
+  static constexpr bool contiguous = false, scattered = NC >= 8;
+};
+
+// (where it is not one site per thread)
 template <typename R, int NC>
 struct ComputeBound<GenExpOp<R, NC>> {
   static constexpr bool value = true;

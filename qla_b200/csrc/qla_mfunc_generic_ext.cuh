@@ -460,4 +460,23 @@ struct GenEigenOp {
   __device__ static void finish(const SiteParams&, const double*) {}
 };
 
+// (measurements beside GenSqrtOp's; expA is exp's arithmetic)
+template <typename R, int NC, int NB>
+struct SitePerThread<GenMInverseOp<R, NC, NB>> {
+  static constexpr bool contiguous = NC >= 4 && !(NC == 4 && NB == 4 && sizeof(R) == 4), scattered = NC >= 4;
+};
+template <typename R, int NC, int WHICH>
+struct SitePerThread<GenMfuncExtOp<R, NC, WHICH>> {
+  static constexpr bool slots = NC == 4 && sizeof(R) == 4 && (WHICH == 1 || WHICH == 2);  // log, expA
+  static constexpr bool contiguous = NC >= 4 && !slots, scattered = contiguous || (NC == 3 && WHICH == 1);
+};
+template <int WHICH>
+struct ComputeBound<GenMfuncExtOp<float, 4, WHICH>> {
+  static constexpr bool value = WHICH == 1 || WHICH == 2;
+};
+template <typename R, int NC, bool HERM>
+struct SitePerThread<GenEigenOp<R, NC, HERM>> {
+  static constexpr bool contiguous = NC >= 4, scattered = NC >= 4;
+};
+
 }  // namespace qlab
