@@ -471,6 +471,12 @@ template <class OP>
 struct SitePerThread {
   static constexpr bool contiguous = false, scattered = false;
 };
+// Operators with slots so large that only three or four warps fit on an SM, where
+// they lose to one site per thread (specialised beside them).
+template <class OP>
+struct FewWarps {
+  static constexpr bool value = false;
+};
 // Operators whose arithmetic hides behind the movement of their records even
 // with half the usual warps (specialised beside them).
 template <class OP>
@@ -556,8 +562,9 @@ __global__ void __launch_bounds__(128, coop_min_blocks<OP>()) site_coop_kernel(c
 // Kernel 3: one site per thread, records read and written where they lie, up to
 // 255 registers a thread.  For operators whose arithmetic on one site outweighs
 // its bytes and needs more registers, or more local memory, than the warps that
-// share shared-memory slots can have (SitePerThread), and for the allocation-free
-// entry point's unaligned calls.  Operators of two inputs load with ld_here: into
+// share shared-memory slots can have (SitePerThread), for scattered calls whose
+// records are too short or too long for those slots (SiteLauncher), and for the
+// allocation-free entry point's unaligned calls.  Operators of two inputs load with ld_here: into
 // local arrays, plain loads of the second record wait for the first one's stores
 // (QLA_DN_M_xeq_M_inverse_M, nc = 8, 23,438 sites: 159 us with __ldg, 237 plain).
 template <class OP>

@@ -242,6 +242,25 @@ struct SiteLauncher {
       check_launch(kernel_id);
   }
 
+  // Scattered calls that the warp-cooperative kernel would slow down: records so
+  // short that neighbouring sites share lines, in fields that fill the GPU, and
+  // operators that leave an SM three or four of its warps (FewWarps), in fields of
+  // more than one round of those.  Measured on gang calls, us, warp-cooperative / one
+  // site per thread: D3 norm2_V on 166,667 sites 9.6 / 6.7, F3 norm2_V on 1.39 M 15.1 /
+  // 13.6, FN re_V_dot_V nc = 2 on 750,000 13.6 / 10.4, but F3 V_dot_V on 1.39 M 28 / 31
+  // and FN norm2_H nc = 2 on 3.1 M 40 / 44; below 65,536 sites a few per cent the other
+  // way.  FN V_xpeq_V nc = 2 on 3.1 M 60 / 50.  DN D_xpeq_M_times_D nc = 8 on 15,000 sites
+  // 48 / 34, on 23,438 52 / 34, but on 1,500 29 / 34; M_xeq_M_times_M on 15,000 96 / 219.
+  static bool coop_loses(const SiteParams& p, int sms) {
+    constexpr int RBMAX = RB[0] > RB[1] ? (RB[0] > RB[2] ? RB[0] : RB[2]) : (RB[1] > RB[2] ? RB[1] : RB[2]);
+    constexpr int SHORT = OP::NACC == 0 ? (StreamsRecords<OP>::value && OB <= 16 ? 32 : 0)
+                          : sizeof(R) == 8 ? 48 : OP::NIN == 1 ? 24 : 16;
+    if (RBMAX <= SHORT) return p.n > 65536;
+    if (!FewWarps<OP>::value) return false;
+    const Shape& sh = coop_shape();
+    return p.n > (long long)sh.blocks * sh.threads * sms;
+  }
+
   // One site per thread, in blocks of 256; of fewer threads (32 at least) while
   // blocks of twice as many would leave SMs without one (QLA_DN_M_veq_invsqrt_M,
   // nc = 8, 3,000 sites: blocks of 256 1,012 us, so 269).
@@ -302,7 +321,7 @@ struct SiteLauncher {
       if (host_result) p.result = rs->result;
     }
 
-    if (per_site) {
+    if (per_site || (scattered && coop_loses(p, sms))) {
       run_per_site(p, kernel_id, sms, rs, host_result, result_bytes);
       return;
     }

@@ -424,6 +424,11 @@ struct ReDotOp {
   __device__ static void finish(const SiteParams& p, const double* tot) { write_real<OUT>(p, tot[0]); }
 };
 
+template <int NCOL, bool ADJA, bool ADJB>
+struct FewWarps<LMultOp<double, 8, NCOL, ADJA, ADJB>> {
+  static constexpr bool value = NCOL == 2 || NCOL == 4;
+};
+
 // operators that only stream records (tile size of small fields)
 template <typename R, int NC, int NCOL, bool ADJA, bool ADJB>
 struct StreamsRecords<LMultOp<R, NC, NCOL, ADJA, ADJB>> {

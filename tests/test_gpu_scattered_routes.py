@@ -76,3 +76,49 @@ def test_scattered_log_and_eigenvalues(qla, lib, dt):
             gang = rng.permutation(n).astype(np.int32)
             getattr(ns_, f"{dest}_xeq_{fname}_M")(x, a, T.to_dev(gang), n)
             assert T.bits_equal(T.to_host(x), T.to_host(v)), (fname, n)
+
+
+@pytest.mark.parametrize("lib,dt", [("FN", np.float32), ("DN", np.float64)])
+def test_scattered_short_and_long_records(qla, cuda, lib, dt):
+    """Gang-index calls around the sizes where they leave the warp-cooperative
+    kernel: V of two colours (65,536 sites; reductions and products), and H and D
+    of eight colours (one round of the few warps that fit)."""
+    rng = np.random.default_rng(321)
+    ns_ = getattr(qla, lib)
+    red = getattr(qla, "DFN" if lib == "FN" else "DN")
+    sms = qla.lib().qlagpu_sm_count()
+    for nc, dest, ncol, sizes in ((2, "V", 1, (65535, 65536, 65537, 70001)),
+                                  (8, "H", 2, (33, 96 * sms, 96 * sms + 1, 128 * sms, 128 * sms + 33)),
+                                  (8, "D", 4, (33, 96 * sms, 96 * sms + 1, 128 * sms, 128 * sms + 33))):
+        ncx, ns = nc * ncol, max(sizes) + 7
+        a, b = T.gaussian_field(rng, ns, nc * nc, dt), T.gaussian_field(rng, ns, ncx, dt)
+        ad, bd = T.to_dev(a), T.to_dev(b)
+        for n in sizes:
+            gang = np.sort(rng.permutation(ns)[:n]).astype(np.int32)
+            gd = T.to_dev(gang)
+            for eq in ("eq", "peq"):
+                r0 = T.gaussian_field(rng, ns, ncx, dt)
+                rd, want = T.to_dev(r0), r0.copy()
+                getattr(ns_, f"{dest}_x{eq}_M_times_{dest}")(nc, rd, ad, bd, gd, n)
+                T.ora_lmult(want, a, b, n, ncol, eq, gang=gang, nc=nc)
+                assert T.bits_equal(T.to_host(rd), want), (nc, dest, eq, n)
+            if dest == "V":
+                exact = T.ora_norm2(b, n, ncx, exact=True, gang=gang)
+                got = red.r_xeq_norm2_V(nc, None, bd, gd, n)
+                assert abs(got - exact) <= 1e-12 * exact, n
+                c = T.gaussian_field(rng, ns, ncx, dt)
+                ed = T.ora_dot(b, c, n, ncx, exact=True, gang=gang)
+                gotd = red.c_xeq_V_dot_V(nc, None, bd, T.to_dev(c), gd, n)
+                assert abs(gotd - ed) <= 1e-12 * max(1.0, abs(ed)) * 4, n
+    assert qla.device_error() == 0
+
+
+@pytest.mark.parametrize("lib,dt,red", [("F3", np.float32, "DF3"), ("D3", np.float64, "D3")])
+@pytest.mark.parametrize("n", [65536, 65537, 100003])
+def test_scattered_vector_reductions(qla, lib, dt, red, n):
+    rng = np.random.default_rng(331 + n)
+    b = T.gaussian_field(rng, n + 5, 3, dt)
+    gang = np.sort(rng.permutation(n + 5)[:n]).astype(np.int32)
+    exact = T.ora_norm2(b, n, 3, exact=True, gang=gang)
+    got = getattr(qla, red).r_xeq_norm2_V(None, T.to_dev(b), T.to_dev(gang), n)
+    assert abs(got - exact) <= 1e-12 * exact
