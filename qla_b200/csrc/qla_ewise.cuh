@@ -484,7 +484,8 @@ __device__ __forceinline__ void ldot_term(Cx<R> ua, Cx<R> vb, double& xr, double
   }
 }
 // the accumulation of one site: x over the elements e in order, from the
-// records a and b (any memory space); blk: row length of the permuted source
+// records a and b (any memory space) of ne numbers; blk: row length of the
+// permuted source
 template <typename R, int KIND>
 __device__ __forceinline__ void ldot_site(const Cx<R>* a, const Cx<R>* b, int ne, int blk, double& xr, double& xi) {
   xr = 0.0;
@@ -499,6 +500,35 @@ __device__ __forceinline__ void ldot_site(const Cx<R>* a, const Cx<R>* b, int ne
   } else {
 #pragma unroll 4
     for (int e = 0; e < ne; e++) ldot_term<R, KIND>(a[e], b[e], xr, xi);
+  }
+}
+// The same for records read where they lie in global memory, where it matters
+// how many loads of a thread are in flight and how many threads share the L1.
+// Measured, us, ldot_site / so: the record length NE known at compile time, D3
+// re_M_dot_pM on 1.39 M sites 143 / 104, F3 re_D_dot_pD on 2.8 M 207 / 179 (but F3
+// norm2_P on 333,333 gang sites 342 / 382, F3 Ma_dot_M on 1.39 M 92 / 111: those stay
+// with ldot_site); N colours not unrolled by hand, DN re_D_dot_D nc = 4 on 390,625 gang
+// sites 111 / 104, M_dot_Ma 110 / 98 (but FN norm2_pD nc = 4 on 375,000 48 / 51).
+template <typename R, int KIND, int NE>
+__device__ __forceinline__ void ldot_scattered(const Cx<R>* a, const Cx<R>* b, int ne, int blk, double& xr,
+                                               double& xi) {
+  constexpr bool permuted = KIND == LD_ADOT || KIND == LD_DOT_AA;
+  if constexpr (NE == 1 || (NE > 0 && !permuted && (KIND != LD_NORM2 || sizeof(R) == 8))) {
+    xr = 0.0;
+    xi = 0.0;
+#pragma unroll 4
+    for (int e = 0; e < NE; e++) ldot_term<R, KIND>(a[e], b[e], xr, xi);
+  } else if (NE == 0 && (permuted ? sizeof(R) == 8 : KIND != LD_NORM2)) {
+    const int rows = permuted ? blk : 1, cols = permuted ? blk : ne;
+    xr = 0.0;
+    xi = 0.0;
+    for (int x = 0; x < rows; x++)
+      for (int y = 0; y < cols; y++) {
+        const int e = x * cols + y, pe = permuted ? y * blk + x : e;
+        ldot_term<R, KIND>(a[KIND == LD_ADOT ? pe : e], b[KIND == LD_DOT_AA ? pe : e], xr, xi);
+      }
+  } else {
+    ldot_site<R, KIND>(a, b, ne, blk, xr, xi);
   }
 }
 
@@ -525,7 +555,7 @@ __device__ __forceinline__ void ldot_store(void* out, long long k, int eqop, dou
 }
 
 // one thread per site, records read where they are (gang or pointer forms)
-template <typename R, int KIND>
+template <typename R, int KIND, int NE>
 __global__ void __launch_bounds__(256) ldot_kernel(const EwParams p, int ne, int blk) {
   overlap_begin();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < p.n;
@@ -534,7 +564,7 @@ __global__ void __launch_bounds__(256) ldot_kernel(const EwParams p, int ne, int
     const Cx<R>* a = rec_ptr<R>(p.b, k, ne);
     const Cx<R>* b = (KIND == LD_NORM2) ? a : rec_ptr<R>(p.c, k, ne);
     double xr, xi;
-    ldot_site<R, KIND>(a, b, ne, blk, xr, xi);
+    ldot_scattered<R, KIND, NE>(a, b, ne, blk, xr, xi);
     ldot_store<R, KIND>(p.out, k, p.eqop, xr, xi);
   }
 }
@@ -648,8 +678,9 @@ __global__ void __launch_bounds__(128) ldot_tile_kernel(const EwParams p, int ne
   }
 }
 
-// ne complex numbers per record, blk: row length of a permuted source
-template <typename R, int KIND>
+// ne complex numbers per record (NE: the same, 0 where it is not known at compile
+// time), blk: row length of a permuted source
+template <typename R, int KIND, int NE>
 inline void run_ldot(const char* kid, int ne, int blk, void* r, Opnd a, Opnd b, const int* gang, int n, int eqop) {
   EwParams p;
   std::memset(&p, 0, sizeof(p));
@@ -680,7 +711,7 @@ inline void run_ldot(const char* kid, int ne, int blk, void* r, Opnd a, Opnd b, 
   } else {
     long long grid = ((long long)n + 255) / 256;
     if (grid > (long long)sms * 16) grid = (long long)sms * 16;
-    launch_kernel(ldot_kernel<R, KIND>, (unsigned)(grid < 1 ? 1 : grid), 256, 0, current_stream(), p, ne, blk);
+    launch_kernel(ldot_kernel<R, KIND, NE>, (unsigned)(grid < 1 ? 1 : grid), 256, 0, current_stream(), p, ne, blk);
   }
   check_launch(kid);
 }
@@ -692,7 +723,7 @@ inline void api_ldot(const char* kid, void* r, Opnd a, Opnd b, const int* gang, 
     set_error(QLAGPU_ERR_NULLPTR, kid, "NULL argument");
     return;
   }
-  run_ldot<R, KIND>(kid, NE, PERM == PERM_P ? 12 : PERM == PERM_M ? 3 : 1, r, a, b, gang, n, eqop);
+  run_ldot<R, KIND, NE>(kid, NE, PERM == PERM_P ? 12 : PERM == PERM_M ? 3 : 1, r, a, b, gang, n, eqop);
 }
 
 }  // namespace qlab

@@ -219,7 +219,7 @@ inline void api_ldot_n(const char* kid, int nc, int ne, int perm, void* r, Opnd 
     set_error(QLAGPU_ERR_NULLPTR, kid, "NULL argument");
     return;
   }
-  run_ldot<R, KIND>(kid, ne, nc_dims(nc, ne, perm).blk, r, a, b, gang, n, eqop);
+  run_ldot<R, KIND, 0>(kid, ne, nc_dims(nc, ne, perm).blk, r, a, b, gang, n, eqop);
 }
 
 // ---------------------------------------------------------------------------
