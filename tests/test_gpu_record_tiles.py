@@ -182,3 +182,19 @@ def test_register_limited_operators_take_smaller_tiles(qla, pc, dt, n):
         assert T.bits_equal(T.to_host(r), want), fname
         getattr(ns_, f"M_veq_{fname}_pM")(r, ptrs, n)
         assert T.bits_equal(T.to_host(r), want[idx]), fname + " pM"
+
+
+@pytest.mark.parametrize("pc", ["F3", "D3"])
+def test_partial_tiles_of_propagators(qla, cuda, pc):
+    """Fields whose last tile of 32 sites is nearly empty, nearly full or the only
+    one, on and off a 16-B boundary (P records: one bulk copy per lane)."""
+    byname = {e["name"]: e for e in qla.manifest()}
+    rng = np.random.default_rng(83)
+    dt = np.float32 if pc == "F3" else np.float64
+    for n in (1, 2, 31, 33, 63, 3000):
+        for short in ("R_veq_re_P_dot_P", "R_vpeq_norm2_P", "C_veq_P_dot_P", "C_vmeq_P_dot_Pa", "C_veq_Pa_dot_P"):
+            e = byname[f"QLA_{pc}_{short}"]
+            ins, idx, gang = T.ewise_inputs(e, rng, dt, n, n)
+            want = T.ewise_oracle(e, ins, idx, gang, n)
+            for off in (0, 8):
+                assert T.bits_equal(_call(qla, cuda, e["name"], [], e, ins, n, off), want), (short, n, off)
