@@ -198,3 +198,29 @@ def test_partial_tiles_of_propagators(qla, cuda, pc):
             want = T.ewise_oracle(e, ins, idx, gang, n)
             for off in (0, 8):
                 assert T.bits_equal(_call(qla, cuda, e["name"], [], e, ins, n, off), want), (short, n, off)
+
+
+@pytest.mark.parametrize("pc,nc", [("F", 3), ("D", 3), ("F3", 3), ("D3", 3), ("FN", 2), ("DN", 2)])
+def test_local_products_of_short_records(qla, cuda, pc, nc):
+    """Records of 8 to 48 B around 65,536 sites, where the longer ones change kernel."""
+    byname = {e["name"]: e for e in qla.manifest()}
+    rng = np.random.default_rng(87 + nc)
+    dt = np.float32 if pc[0] == "F" else np.float64
+    L = qla.lib()
+    for n in (65535, 65536, 65537):
+        for letter in ("C",) if len(pc) == 1 else ("V", "H"):
+            ne = {"C": 1, "V": nc, "H": 2 * nc}[letter]
+            a, b = T.gaussian_field(rng, n, ne, dt), T.gaussian_field(rng, n, ne, dt)
+            x, y = a.astype(np.float64), b.astype(np.float64)
+            lead = [nc] if pc[1:] == "N" else []
+            for short, want in ((f"R_veq_norm2_{letter}", (x, x)), (f"R_veq_re_{letter}_dot_{letter}", (x, y))):
+                assert f"QLA_{pc}_{short}" in byname
+                r = T.to_dev(np.zeros(n, dt))
+                keep = [T.to_dev(a), T.to_dev(b)]
+                args = [T.ptr_dev(r), T.ptr_dev(keep[0])] + ([T.ptr_dev(keep[1])] if "re_" in short else [])
+                getattr(L, f"QLA_{pc}_{short}")(*lead, *args, n)
+                s = np.zeros(n)
+                for e in range(ne):  # the reference's order, in double
+                    s = s + (want[0][:, 2 * e] * want[1][:, 2 * e] + want[0][:, 2 * e + 1] * want[1][:, 2 * e + 1])
+                assert T.bits_equal(T.to_host(r), s.astype(dt)), (pc, short, n)
+    qla.check("short records")
