@@ -330,6 +330,12 @@ struct EwAdjointOp {
   __device__ static void finish(const SiteParams&, const double*) {}
 };
 
+// Fields of fewer sites than this stay with one thread per element: the tiles'
+// pipeline takes longer to fill than such a field to move (us, per element / tiles:
+// QLA_F3_M_veq_Ca_times_Ma on 3,000 sites 3.5 / 4.1, on 30,000 4.6 / 4.7, on 666,666 22
+// / 14; M_veq_V_times_Va on 10,000 3.7 / 4.5, on 30,000 4.5 / 4.2).
+inline bool engine_pays(int n) { return n > 128LL * device_sm_count(); }
+
 // host side: SCAL_ARG is a pointer to the constant (host or device memory)
 // for SC_CONST, ignored otherwise
 template <typename R, int NE, int SHAPE, int PERM, int SCAL, bool SREAL>
@@ -361,7 +367,7 @@ inline void api_ew(const char* kid, void* r, const void* scal, Opnd s, Opnd b, O
     }
   }
   if constexpr (PERM == PERM_M && NE == 9 && !TWO && !(SCAL == SC_FIELD && SREAL)) {
-    if (gang == nullptr && b.mode == OM_CONTIG && aligned16(r) && aligned16(b.base) &&
+    if (gang == nullptr && engine_pays(n) && b.mode == OM_CONTIG && aligned16(r) && aligned16(b.base) &&
         (SCAL != SC_FIELD || (s.mode == OM_CONTIG && aligned16(s.base)))) {
       SiteParams q = make_params(n, eqop);
       q.in[0] = SCAL == SC_FIELD ? s : b;
@@ -439,8 +445,8 @@ inline void api_outer(const char* kid, void* r, Opnd a, Opnd b, const int* gang,
     set_error(QLAGPU_ERR_NULLPTR, kid, "NULL argument");
     return;
   }
-  if (gang == nullptr && a.mode == OM_CONTIG && b.mode == OM_CONTIG && aligned16(r) && aligned16(a.base) &&
-      aligned16(b.base)) {
+  if (gang == nullptr && engine_pays(n) && a.mode == OM_CONTIG && b.mode == OM_CONTIG && aligned16(r) &&
+      aligned16(a.base) && aligned16(b.base)) {
     api_map<OuterOp<R>>(kid, r, a, b, gang, n, eqop);
     return;
   }

@@ -224,3 +224,18 @@ def test_local_products_of_short_records(qla, cuda, pc, nc):
                     s = s + (want[0][:, 2 * e] * want[1][:, 2 * e] + want[0][:, 2 * e + 1] * want[1][:, 2 * e + 1])
                 assert T.bits_equal(T.to_host(r), s.astype(dt)), (pc, short, n)
     qla.check("short records")
+
+
+@pytest.mark.parametrize("pc", ["F3", "D3"])
+def test_adjoint_and_outer_forms_change_kernel_with_size(qla, cuda, pc):
+    byname = {e["name"]: e for e in qla.manifest()}
+    rng = np.random.default_rng(67)
+    dt = np.float32 if pc == "F3" else np.float64
+    top = 128 * qla.lib().qlagpu_sm_count()
+    for n in (top, top + 1, top + 33):
+        for short in ADJOINT + ["M_veq_V_times_Va", "M_vmeq_V_times_Va"]:
+            e = byname[f"QLA_{pc}_{short}"]
+            ins, idx, gang = T.ewise_inputs(e, rng, dt, n, n)
+            want = T.ewise_oracle(e, ins, idx, gang, n)
+            for off in (0, 8):
+                assert T.bits_equal(_call(qla, cuda, e["name"], [], e, ins, n, off), want), (short, n, off)
