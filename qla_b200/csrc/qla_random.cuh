@@ -514,10 +514,22 @@ template <typename R, int MODE>
 inline void rng_launch_fill(const RngParams& p) {
   // (the tile kernel writes records in 8-B pieces)
   if (p.gang == nullptr && p.s.mode == OM_CONTIG &&
-      (p.nreal == 1 || (reinterpret_cast<uintptr_t>(p.out) & 7u) == 0))
+      (p.nreal == 1 || (reinterpret_cast<uintptr_t>(p.out) & 7u) == 0)) {
     launch_kernel(rng_tile_kernel<R, MODE>, (unsigned)((p.n + 127) / 128), 128, 0, current_stream(), p);
-  else
-    launch_kernel(rng_fill_kernel<R, MODE>, rng_grid(p.n, 128), 128, 0, current_stream(), p);
+    return;
+  }
+  // Scattered states: a thread writes its record 4 or 8 B at a time, and the lines of
+  // the records in progress should stay in the L2 until they are whole.  In fields
+  // larger than the L2 (126 MB; a gang index may touch twice what it counts) six blocks
+  // an SM run, else sixteen.  Measured, us, sixteen / six: DN D_veq_gaussian_pS nc = 2 on
+  // 750,000 sites 127 / 98, FN D_xeq_gaussian_S nc = 2 on 750,000 129 / 106, D3
+  // D_xeq_gaussian_S on 694,000 278 / 243; but D3 D_xeq on 166,667 (78 MB) 39 / 43.
+  unsigned grid = rng_grid(p.n, 128);
+  if ((double)p.n * (p.nreal * (double)sizeof(R) + 44.0) * (p.gang ? 2.0 : 1.0) > 126e6) {
+    const unsigned cap = 6u * (unsigned)device_sm_count();
+    if (grid > cap) grid = cap;
+  }
+  launch_kernel(rng_fill_kernel<R, MODE>, grid, 128, 0, current_stream(), p);
 }
 
 // r (nreal reals per record of R) = uniform (gauss 0) or gaussian deviates
