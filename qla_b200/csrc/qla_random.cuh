@@ -12,11 +12,10 @@
 // double (default) or MILC's polar method (QLA_use_milc_gaussian != 0, the
 // spare deviate kept in the state's addend / scale words), rounded to float.
 // The polar method's double log and sqrt are CUDA's; Box-Muller's log, sqrt and
-// cos are written out below for the arguments that a 24-bit deviate gives (over
-// all of them log within 1.4 ulp, sqrt 0.5 and cos 1.5 ulp of the double); a
-// last-place difference from the host libm changes the float result only when
-// it falls within that distance of a float rounding boundary (none of 2^24
-// pairs of deviates).
+// cos are written out below for the arguments that a 24-bit deviate gives.  A
+// difference of a few units in the last place of the double from the host libm
+// changes the float result only where the double lies that near the midpoint of
+// two floats (tests/test_gpu_box_muller.py: every radius, every angle).
 //
 // Fills give each thread one site (the state is sequential within a site) and
 // generate the record's values in the reference's order: for each complex
