@@ -53,7 +53,9 @@ unsigned qlagpu_device_error(int clear);
 
 /* autotuner: launch shape (threads per block = sites per tile: 64/128/256,
  * pipeline stages: 2..8) for one kernel id, as reported by
- * qla_b200.tune; qlagpu_tune_clear() restores the built-in heuristic */
+ * qla_b200.tune; qlagpu_tune_clear() restores the built-in heuristic.  It
+ * applies where the call runs tiles of that kernel: small fields take 64-site
+ * tiles of two stages, gang-index and unaligned calls other kernels */
 int qlagpu_tune_set(const char *kernel_id, int threads, int stages);
 void qlagpu_tune_clear(void);
 

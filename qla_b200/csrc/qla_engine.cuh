@@ -13,8 +13,9 @@
 //
 // A second, warp-cooperative kernel runs the gang-index `x` variants, whose
 // every operand is scattered, and any call whose pointers are not 16-B
-// aligned (bulk copies require 16-B alignment).  Both kernels share the
-// per-site code, so their results are identical.
+// aligned (bulk copies require 16-B alignment); a third runs one site per
+// thread, for operators and calls that either of these would slow down.  The
+// kernels share the per-site code, so their results are identical.
 //
 // An operator type OP provides:
 //   using R;                               site real type (float/double)
