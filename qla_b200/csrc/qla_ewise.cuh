@@ -705,13 +705,14 @@ inline void run_ldot(const char* kid, int ne, int blk, void* r, Opnd a, Opnd b, 
   const size_t warp_bytes = 128u + NOP * 32u * (size_t)ldot_slot(rb);
   const int sms = device_sm_count();
   // Records that neighbouring lanes read from the same lines need no staging: up to
-  // 24 B always, up to 48 B in small fields, where the copies' latency counts, and up
-  // to 32 B for norms in double.  Measured, us, tiles / one site per thread: F norm2_C on
+  // 24 B always, up to 48 B in small fields, where the copies' latency counts; in double
+  // 48 B always, and norms of 32 B.  Measured, us, tiles / one site per thread: F norm2_C on
   // 666,666 sites 5.6 / 4.2, F3 norm2_V 6.4 / 3.7, FN norm2_V nc = 2 on 1.5 M 11.6 / 6.1,
-  // on 30,000 4.6 / 3.5, DN norm2_V nc = 2 on 750,000 6.8 / 5.5, D3 V_dot_V on 30,000
-  // 4.4 / 3.5; but FN H_dot_H nc = 2 (32 B) on 1.5 M 17 / 27, F3 norm2_H (48 B) on 666,666
-  // 7.1 / 7.5.
-  const bool near = rb <= 24u || (rb <= 48u && n <= 65536) || (KIND == LD_NORM2 && sizeof(R) == 8 && rb <= 32u);
+  // on 30,000 4.6 / 3.5, DN norm2_V nc = 2 on 750,000 6.8 / 5.5, D3 V_dot_V on 333,333 7.6 /
+  // 5.3, on 30,000 4.4 / 3.5; but FN H_dot_H nc = 2 (32 B) on 1.5 M 17 / 27, DN V_dot_V
+  // nc = 2 (32 B) on 750,000 9.1 / 9.9, F3 norm2_H (48 B) on 666,666 7.1 / 7.5.
+  const bool near = rb <= 24u || (rb <= 48u && n <= 65536) ||
+                    (sizeof(R) == 8 && (rb == 48u || (KIND == LD_NORM2 && rb <= 32u)));
   // (records too long for one warp's slots -- P of many colours -- go direct)
   if (gang == nullptr && a.mode == OM_CONTIG && (KIND == LD_NORM2 || b.mode == OM_CONTIG) &&
       !near && warp_bytes <= 200u * 1024u) {
